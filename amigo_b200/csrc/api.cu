@@ -139,7 +139,7 @@ struct b200ldl_handle {
   DevPlan plan{};
 
   // device state
-  DevBuf<int> d_f, d_fs, d_npiv, d_ndel, d_L_ld, d_cb_ld, d_ivars, d_err, d_inertia;
+  DevBuf<int> d_f, d_fs, d_npiv, d_ndel, d_L_ld, d_cb_ld, d_ivars, d_err, d_inertia, d_done, d_ticket;
   DevBuf<int64_t> d_fv_off, d_L_off, d_cb_off, d_u_off;
   DevBuf<double> d_dpool, d_flops, d_upool, d_vals, d_diag, d_x;
   DevBuf<unsigned long long> d_used;
@@ -471,6 +471,8 @@ void upload_plan(b200ldl_t h) {
   CK(h->d_L_off.alloc(nn));
   CK(h->d_cb_off.alloc(nn));
   CK(h->d_u_off.alloc(nn));
+  CK(h->d_done.alloc(nn));
+  CK(h->d_ticket.alloc(h->num_levels));
   CK(h->d_err.alloc(4));
   CK(h->d_inertia.alloc(2));
   CK(h->d_flops.alloc(kWork));
@@ -498,6 +500,7 @@ void bind_state(b200ldl_t h) {
   st.used = h->d_used.ptr;
   st.icap = h->icap;
   st.dcap = h->dcap;
+  st.done = h->d_done.ptr;
   st.err = h->d_err.ptr;
   st.inertia = h->d_inertia.ptr;
   st.flops = h->d_flops.ptr;
@@ -559,17 +562,35 @@ void run_factor_once(b200ldl_t h, const double* vals, const double* diag, bool m
     CK(cudaMemsetAsync(h->d_inertia.ptr, 0, 2 * sizeof(int), h->stream));
     CK(cudaMemsetAsync(h->d_flops.ptr, 0, kWork * sizeof(double), h->stream));
     CK(cudaMemsetAsync(h->d_ndel.ptr, 0, sizeof(int) * std::max(1, h->sym.num_nodes), h->stream));
+    CK(cudaMemsetAsync(h->d_done.ptr, 0, sizeof(int) * std::max(1, h->sym.num_nodes), h->stream));
+    CK(cudaMemsetAsync(h->d_ticket.ptr, 0, sizeof(int) * std::max(1, h->num_levels), h->stream));
     for (int l = 0; l < h->num_levels; l++) {
       const int b = h->level_ptr[l];
-      const int cnt = h->level_ptr[l + 1] - b;
+      // consecutive levels without big fronts share a launch: twice the
+      // widest level's CTAs, so that fronts of the next level load their own
+      // entries while this level's are factored, and no more than can be
+      // resident
+      int l1 = l + 1, fcap = h->level_fcap[l], width = h->level_ptr[l + 1] - b;
+      if (!h->level_big[l])
+        for (; l1 < h->num_levels && !h->level_big[l1]; l1++) {
+          fcap = std::max(fcap, h->level_fcap[l1]);
+          width = std::max(width, h->level_ptr[l1 + 1] - h->level_ptr[l1]);
+        }
+      const int cnt = h->level_ptr[l1] - b;
+      const bool run = l1 > l + 1;
       if (h->level_big[l])
         CK(cudaMemsetAsync(h->d_big_meta.ptr, 0, kBigMeta * sizeof(int), h->stream));
       h->prof.begin(h->stream);
-      launch_factor_level(h->plan, h->st, h->d_level_nodes.ptr + b, cnt, h->level_fcap[l],
-                          h->level_big[l], prm, h->stream, vals, diag);
+      launch_factor_level(h->plan, h->st, h->d_level_nodes.ptr + b, cnt,
+                          run ? h->d_ticket.ptr + l : nullptr,
+                          run ? std::min({cnt, 2 * width, 148 * 4}) : cnt, fcap, h->level_big[l],
+                          prm, h->stream, vals, diag);
       h->prof.end(kPhFront, h->stream, 1);
       CK(cudaGetLastError());
-      if (!h->level_big[l]) continue;
+      if (!h->level_big[l]) {
+        l = l1 - 1;
+        continue;
+      }
       int meta[kBigMeta];
       CK(cudaMemcpyAsync(meta, h->d_big_meta.ptr, kBigMeta * sizeof(int), cudaMemcpyDeviceToHost,
                          h->stream));
@@ -633,6 +654,7 @@ void run_factor_once(b200ldl_t h, const double* vals, const double* diag, bool m
       }
       return;
     }
+    if (err[0] & 8) throw std::runtime_error("a front's children did not complete in time");
     if (err[0] & 4) {
       // a front went big in a level not prepared for one: every level whose
       // bound allows one is prepared

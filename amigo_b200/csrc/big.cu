@@ -774,6 +774,7 @@ __global__ void big_finalize_kernel(DevState s, int nbig, int cholesky) {
     s.cb_off[node] = B.doff + (long long)npiv * (B.f + 1);
     s.cb_ld[node] = B.f;
   }
+  s.done[node] = 1;
   s.u_off[node] = (long long)atomicAdd(s.used + 2, (unsigned long long)m);
   if (!cholesky) {
     atomicAdd(s.inertia, B.npos);
