@@ -66,6 +66,40 @@ struct CudaError : std::runtime_error {
     if (e__ != cudaSuccess) throw CudaError(e__, #call); \
   } while (0)
 
+// Words of pinned host memory that kernels write a failure to, one per handle
+// that has solved. A pinned allocation takes longer than a small solve, so
+// they are handed out of pages that the process keeps (one page serves 1024
+// handles at a time).
+class HostWords {
+ public:
+  int* take() {
+    std::lock_guard<std::mutex> lock(mu_);
+    if (free_.empty()) {
+      int* page = nullptr;
+      CK(cudaHostAlloc(&page, kPerPage * sizeof(int), cudaHostAllocPortable));
+      for (int i = 0; i < kPerPage; i++) free_.push_back(page + i);
+    }
+    int* w = free_.back();
+    free_.pop_back();
+    *w = 0;
+    return w;
+  }
+  void give(int* w) {
+    std::lock_guard<std::mutex> lock(mu_);
+    free_.push_back(w);
+  }
+
+ private:
+  static constexpr int kPerPage = 1024;
+  std::mutex mu_;
+  std::vector<int*> free_;
+};
+
+HostWords& host_words() {
+  static HostWords* words = new HostWords;  // outlives every handle
+  return *words;
+}
+
 }  // namespace
 
 struct b200ldl_handle {
@@ -163,13 +197,23 @@ struct b200ldl_handle {
   std::vector<int> level_fmax;
   // solve schedule of the last factorization: per level, the supernodes for
   // the one-CTA kernels then those for the cluster kernels
-  std::vector<int> solve_ptr;    // [2 * levels + 1]
+  // of consecutive levels, the supernodes for the one-CTA kernel (from
+  // `first` on), then the last of these levels' for the cluster kernels
+  struct SolveRun {
+    int first = 0, count = 0, fmax = 1, width = 0, levels = 0;
+    int big_count = 0, big_fmax = 1;
+  };
+  std::vector<SolveRun> solve_runs;
   std::vector<int> solve_nodes;  // host copy of d_solve_nodes
-  std::vector<int> solve_fmax;   // [2 * levels]: largest front of each list
-  DevBuf<int> d_solve_nodes;
+  DevBuf<int> d_solve_nodes, d_parent, d_fdone, d_bdone, d_solve_ticket;
+  int solve_epoch = 0;        // solves so far (the flags' values follow it)
+  int* solve_fail = nullptr;  // pinned host memory
   Prof prof;
   double flops4[kWork] = {};
   double sum_delayed = 0.0;
+  ~b200ldl_handle() {
+    if (solve_fail) host_words().give(solve_fail);
+  }
 };
 
 namespace {
@@ -472,6 +516,12 @@ void upload_plan(b200ldl_t h) {
   CK(h->d_cb_off.alloc(nn));
   CK(h->d_u_off.alloc(nn));
   CK(h->d_done.alloc(nn));
+  CK(h->d_parent.upload(s.parent));
+  CK(h->d_fdone.alloc(nn));
+  CK(h->d_bdone.alloc(nn));
+  CK(cudaMemsetAsync(h->d_fdone.ptr, 0, h->d_fdone.count * sizeof(int), h->stream));
+  CK(cudaMemsetAsync(h->d_bdone.ptr, 0, h->d_bdone.count * sizeof(int), h->stream));
+  if (!h->solve_fail) h->solve_fail = host_words().take();
   CK(h->d_ticket.alloc(h->num_levels));
   CK(h->d_err.alloc(4));
   CK(h->d_inertia.alloc(2));
@@ -703,27 +753,41 @@ void level_fronts(b200ldl_t h) {
   std::vector<int> f(nn);
   CK(cudaMemcpy(f.data(), h->d_f.ptr, nn * sizeof(int), cudaMemcpyDeviceToHost));
   h->level_fmax.assign(h->num_levels, 1);
-  h->solve_ptr.assign(2 * h->num_levels + 1, 0);
-  h->solve_fmax.assign(2 * h->num_levels, 1);
+  h->solve_runs.clear();
   h->solve_nodes.clear();
   int m = 1;
+  b200ldl_handle::SolveRun run;
+  std::vector<int> big;
   for (int l = 0; l < h->num_levels; l++) {
-    for (int pass = 0; pass < 2; pass++) {
-      h->solve_ptr[2 * l + pass] = (int)h->solve_nodes.size();
-      for (int q = h->level_ptr[l]; q < h->level_ptr[l + 1]; q++) {
-        const int node = h->hp_level_nodes[q];
-        const int fn = f[node];
-        const bool big = fn >= kSolveBigFront && solve_big_fits(fn);
-        if (big != (pass == 1)) continue;
-        h->solve_nodes.push_back(node);
-        h->solve_fmax[2 * l + pass] = std::max(h->solve_fmax[2 * l + pass], fn);
-        if (!big) m = std::max(m, fn);
+    big.clear();
+    int width = 0;
+    for (int q = h->level_ptr[l]; q < h->level_ptr[l + 1]; q++) {
+      const int node = h->hp_level_nodes[q];
+      const int fn = f[node];
+      h->level_fmax[l] = std::max(h->level_fmax[l], fn);
+      if (fn >= kSolveBigFront && solve_big_fits(fn)) {
+        big.push_back(node);
+        run.big_fmax = std::max(run.big_fmax, fn);
+        continue;
       }
+      h->solve_nodes.push_back(node);
+      run.fmax = std::max(run.fmax, fn);
+      width++;
     }
-    for (int q = h->level_ptr[l]; q < h->level_ptr[l + 1]; q++)
-      h->level_fmax[l] = std::max(h->level_fmax[l], f[h->hp_level_nodes[q]]);
+    run.count += width;
+    run.width = std::max(run.width, width);
+    run.levels += width > 0;
+    m = std::max(m, run.fmax);
+    if (!big.empty() || l + 1 == h->num_levels) {
+      h->solve_nodes.insert(h->solve_nodes.end(), big.begin(), big.end());
+      run.big_count = (int)big.size();
+      h->solve_runs.push_back(run);
+      run = b200ldl_handle::SolveRun();
+      run.first = (int)h->solve_nodes.size();
+    }
   }
-  h->solve_ptr[2 * h->num_levels] = (int)h->solve_nodes.size();
+  const size_t tickets = 2 * std::max<size_t>(1, h->solve_runs.size());
+  if (h->d_solve_ticket.count < tickets) CK(h->d_solve_ticket.alloc(tickets));
   if (h->d_solve_nodes.count < h->solve_nodes.size())
     CK(h->d_solve_nodes.alloc(h->solve_nodes.size()));
   if (!h->solve_nodes.empty())
@@ -732,37 +796,73 @@ void level_fronts(b200ldl_t h) {
   h->fmax = m;  // largest front left to the one-CTA kernels
 }
 
+// x <- K^-1 x, in chunks of the right-hand sides that a launch takes. The
+// launches are asynchronous; finish_solve waits for them.
 void run_solve(b200ldl_t h, int nrhs, double* x, int ldx) {
   if (h->fmax == 0) level_fronts(h);
-  if (solve_rhs_chunk(h->fmax, 1) < 1)
-    throw std::runtime_error("front too large for the solve kernels");
+  const int chunk = solve_rhs_chunk(h->fmax, nrhs);
+  if (chunk < 1) throw std::runtime_error("front too large for the solve kernels");
   const size_t need = (size_t)h->used[2] * nrhs;
   if (h->d_upool.count < need) CK(h->d_upool.alloc(need));
-  const int* nodes = h->d_solve_nodes.ptr;
-  cudaError_t err = cudaSuccess;
-  for (int l = 0; l < h->num_levels; l++) {
-    const int s0 = h->solve_ptr[2 * l], s1 = h->solve_ptr[2 * l + 1];
-    const int s2 = h->solve_ptr[2 * l + 2];
-    h->prof.begin(h->stream);
-    int nl = launch_forward_level(h->plan, h->st, nodes + s0, s1 - s0, x, ldx, nrhs,
-                                  h->d_upool.ptr, h->solve_fmax[2 * l], h->stream);
-    nl += launch_forward_big(h->plan, h->st, nodes + s1, s2 - s1, x, ldx, nrhs, h->d_upool.ptr,
-                             h->solve_fmax[2 * l + 1], h->stream, &err);
-    CK(err);
-    h->prof.end(kPhFwd, h->stream, nl);
-  }
-  for (int l = h->num_levels - 1; l >= 0; l--) {
-    const int s0 = h->solve_ptr[2 * l], s1 = h->solve_ptr[2 * l + 1];
-    const int s2 = h->solve_ptr[2 * l + 2];
-    h->prof.begin(h->stream);
-    int nl = launch_backward_level(h->plan, h->st, nodes + s0, s1 - s0, x, ldx, nrhs,
-                                   h->solve_fmax[2 * l], h->stream);
-    nl += launch_backward_big(h->plan, h->st, nodes + s1, s2 - s1, x, ldx, nrhs,
-                              h->solve_fmax[2 * l + 1], h->stream, &err);
-    CK(err);
-    h->prof.end(kPhBwd, h->stream, nl);
+  const int nruns = (int)h->solve_runs.size();
+  // one launch for both sweeps where no supernode needs a cluster
+  const bool both = nruns == 1 && h->solve_runs[0].big_count == 0;
+  for (int r0 = 0; r0 < nrhs; r0 += chunk) {
+    const int nr = std::min(chunk, nrhs - r0);
+    h->solve_epoch++;
+    CK(cudaMemsetAsync(h->d_solve_ticket.ptr, 0, 2 * std::max(1, nruns) * sizeof(int),
+                       h->stream));
+    // the run's one-CTA supernodes and its cluster supernodes. CTAs of a run
+    // of several levels: twice the widest level, so that a level's
+    // supernodes load while the one before is solved; not many more than are
+    // resident
+    auto span = [&](int q, bool big, int ticket) {
+      const auto& r = h->solve_runs[q];
+      SolveSpan sp{};
+      sp.nodes = h->d_solve_nodes.ptr + r.first + (big ? r.count : 0);
+      sp.count = big ? r.big_count : r.count;
+      sp.fmax = big ? r.big_fmax : r.fmax;
+      sp.ticket = (r.levels > 1 || both) ? h->d_solve_ticket.ptr + ticket : nullptr;
+      sp.grid = sp.ticket ? std::min({sp.count, 2 * r.width, 148 * 4}) : sp.count;
+      sp.parent = h->d_parent.ptr;
+      sp.fdone = h->d_fdone.ptr;
+      sp.bdone = h->d_bdone.ptr;
+      sp.epoch = h->solve_epoch;
+      sp.fail = h->d_err.ptr + 3;
+      sp.host_fail = h->solve_fail;
+      return sp;
+    };
+    for (int q = 0; q < nruns; q++) {
+      h->prof.begin(h->stream);
+      launch_solve(h->plan, h->st, span(q, false, q), both ? 3 : 1, x, ldx, nrhs, r0, nr,
+                   h->d_upool.ptr, h->stream);
+      CK(launch_forward_big(h->plan, h->st, span(q, true, q), x, ldx, nrhs, r0, nr,
+                            h->d_upool.ptr, h->stream));
+      h->prof.end(kPhFwd, h->stream,
+                  (h->solve_runs[q].count > 0) + (h->solve_runs[q].big_count > 0));
+    }
+    for (int q = both ? -1 : nruns - 1; q >= 0; q--) {
+      h->prof.begin(h->stream);
+      CK(launch_backward_big(h->plan, h->st, span(q, true, nruns + q), x, ldx, r0, nr,
+                             h->stream));
+      launch_solve(h->plan, h->st, span(q, false, nruns + q), 2, x, ldx, nrhs, r0, nr,
+                   h->d_upool.ptr, h->stream);
+      h->prof.end(kPhBwd, h->stream,
+                  (h->solve_runs[q].count > 0) + (h->solve_runs[q].big_count > 0));
+    }
   }
   CK(cudaGetLastError());
+}
+
+// Wait for the launches of run_solve.
+void finish_solve(b200ldl_t h) {
+  CK(cudaStreamSynchronize(h->stream));
+  h->prof.collect();
+  if (h->solve_fail && *((volatile int*)h->solve_fail)) {
+    *h->solve_fail = 0;
+    CK(cudaMemsetAsync(h->d_err.ptr + 3, 0, sizeof(int), h->stream));
+    throw std::runtime_error("a supernode's neighbours were not solved in time");
+  }
 }
 
 template <typename F>
@@ -833,8 +933,7 @@ void refine_impl(b200ldl_t h, const double* vals, const double* diag, int nrhs, 
       max_it_done = std::max(max_it_done, it);
     }
     CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(h->stream));
-    h->prof.collect();
+    finish_solve(h);
     if (iters_out) *iters_out = max_it_done;
     h->last_iters = max_it_done;
     h->last_berr = worst;
@@ -1133,8 +1232,7 @@ static void solve_inplace(b200ldl_t h, int nrhs, double* x, int ldx) {
     launch_copy_cols(h->n, nrhs, h->d_rhs_tmp.ptr, h->n, x, ldx, h->stream);
   }
   run_solve(h, nrhs, x, ldx);
-  CK(cudaStreamSynchronize(h->stream));
-  h->prof.collect();
+  finish_solve(h);
 }
 
 int b200ldl_solve(b200ldl_t h, int nrhs, double* x, int ldx) {

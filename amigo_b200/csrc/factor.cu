@@ -1085,10 +1085,6 @@ __device__ void register_big(const DevPlan& p, const DevState& s, const FactorPa
   }
 }
 
-// Spin limit of a wait for a child (several seconds; a wait normally takes
-// microseconds).
-constexpr int kWaitPolls = 1 << 23;
-
 // kMax: row chunks of the largest front the launch may meet on chip, or
 // kGeneral. CTAs per SM: what the registers of the largest front allow.
 //
@@ -1139,18 +1135,7 @@ __global__ void __launch_bounds__(kFactorThreads, kMax == 1 ? 4 : kMax == 2 ? 3 
         int nd = 0, fail = 0;
         for (int c = kb + lane; c < ke; c += 32) {
           const int ch = p.kids[c];
-          if (ticket) {
-            const volatile int* flag = s.done + ch;
-            int polls = 0;
-            while (*flag == 0) {
-              if (*((volatile int*)s.err) != 0 || ++polls > kWaitPolls) {
-                fail = 1;
-                if (polls > kWaitPolls) atomicOr(s.err, 8);
-                break;
-              }
-            }
-            __threadfence();  // the child's data after its flag
-          }
+          if (ticket && !wait_flag(s.done + ch, 1, s.err, 8)) fail = 1;
           nd += __ldcg(s.ndel + ch);
         }
         nd = __reduce_add_sync(0xffffffffu, nd);
@@ -1348,8 +1333,7 @@ __global__ void __launch_bounds__(kFactorThreads, kMax == 1 ? 4 : kMax == 2 ? 3 
     }
     __syncthreads();
     if (tid == 0) {
-      __threadfence();  // the front's data before its flag
-      *((volatile int*)(s.done + node)) = 1;
+      flag_set(s.done + node, 1);
       s.u_off[node] = (long long)atomicAdd(s.used + 2, (unsigned long long)m);
       if (!prm.cholesky) {
         atomicAdd(s.inertia, o.npos);

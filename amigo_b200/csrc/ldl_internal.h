@@ -152,7 +152,8 @@ struct DevState {
                     // above its launch's on-chip size, 4: a big front in a
                     // level not prepared for one, 8: a wait for a child was
                     // given up), [1] node of first error,
-                    // [2] completion ticket of the trailing-update launch
+                    // [2] completion ticket of the trailing-update launch, [3] a solve's
+                    // wait was given up
   int* inertia;     // [2] pos, neg
   double* flops;    // [kWork] executed flops: [0] all fronts, [1] big panels,
                     // (a-posteriori panels: [5] panels, [6] pivots rejected by
@@ -181,6 +182,38 @@ struct DevState {
   const long long* asm_src;
   const double* asm_blocks;
 };
+
+// Completion flags between CTAs of a launch. A flag is stored after a CTA
+// barrier, with release, so that it orders the whole CTA's writes before it;
+// a reader that sees it and then acquires sees them.
+__device__ __forceinline__ void flag_set(int* flag, int value) {
+  asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(flag), "r"(value) : "memory");
+}
+__device__ __forceinline__ int flag_get(const int* flag) {
+  int v;
+  asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
+  return v;
+}
+
+// Polls the flag until it is at least `value`; false after kWaitPolls polls
+// (several seconds; a wait normally takes microseconds) or once *fail is set,
+// which whoever gives up sets to `code`. Both are in device memory: a read of
+// host memory in the loop would hold up the release of every flag on the SM
+// (a CTA's fence waits for the SM's loads; 20 ms instead of 1.7 for the
+// backward sweep of the 64 x 64 plane-stress system). The polls are relaxed
+// and the acquire comes once, since an acquiring load empties the SM's L1.
+constexpr int kWaitPolls = 1 << 23;
+__device__ __forceinline__ bool wait_flag(const int* flag, int value, int* fail, int code) {
+  for (int polls = 0; flag_get(flag) < value; polls++) {
+    if (polls > kWaitPolls) {
+      *((volatile int*)fail) = code;
+      return false;
+    }
+    if ((polls & 255) == 255 && *((volatile int*)fail) != 0) return false;
+  }
+  asm volatile("fence.acq_rel.gpu;" ::: "memory");
+  return true;
+}
 
 // The CSR value of entry e: from the values, or assembled from the element
 // blocks in the order of the assembly kernel (assembly.cu), so that a front
@@ -277,13 +310,22 @@ constexpr int kSolveThreads = 256;
 // (0 if even one does not fit in shared memory).
 int solve_rhs_chunk(int fmax, int nrhs);
 
-int launch_forward_level(const DevPlan& p, const DevState& s,
-                         const int* level_nodes, int count, double* x,
-                         int ldx, int nrhs, double* upool, int fmax,
-                         cudaStream_t stream);
-int launch_backward_level(const DevPlan& p, const DevState& s,
-                          const int* level_nodes, int count, double* x,
-                          int ldx, int nrhs, int fmax, cudaStream_t stream);
+// The supernodes of one solve launch: those of one or more consecutive levels
+// that take a CTA each, in level order.
+struct SolveSpan {
+  const int* nodes;
+  int count, fmax, grid;
+  int* ticket;        // a zeroed counter when they are of several levels (or of
+                      // both sweeps), else nullptr and grid = count
+  const int* parent;  // [num_nodes], -1 for roots
+  int *fdone, *bdone;  // [num_nodes] progress flags of the two sweeps
+  int epoch;          // number of the solve; the flags of earlier ones are smaller
+  int* fail;          // device memory, set when a wait was given up
+  int* host_fail;     // and host memory
+};
+// sweeps: 1 forward, 2 backward, 3 both in one launch
+void launch_solve(const DevPlan& p, const DevState& s, const SolveSpan& sp, int sweeps, double* x,
+                  int ldx, int nrhs, int r0, int nr, double* upool, cudaStream_t stream);
 cudaError_t configure_solve_kernels();
 
 // Supernodes with fronts of at least kSolveBigFront rows are solved by a
@@ -291,12 +333,11 @@ cudaError_t configure_solve_kernels();
 constexpr int kSolveBigFront = 1024;
 bool solve_big_fits(int f);
 cudaError_t configure_solve_big_kernels();
-int launch_forward_big(const DevPlan& p, const DevState& s, const int* nodes, int count,
-                       double* x, int ldx, int nrhs, double* upool, int fmax,
-                       cudaStream_t stream, cudaError_t* err);
-int launch_backward_big(const DevPlan& p, const DevState& s, const int* nodes, int count,
-                        double* x, int ldx, int nrhs, int fmax, cudaStream_t stream,
-                        cudaError_t* err);
+cudaError_t launch_forward_big(const DevPlan& p, const DevState& s, const SolveSpan& sp, double* x,
+                               int ldx, int nrhs, int r0, int nr, double* upool,
+                               cudaStream_t stream);
+cudaError_t launch_backward_big(const DevPlan& p, const DevState& s, const SolveSpan& sp,
+                                double* x, int ldx, int r0, int nr, cudaStream_t stream);
 
 // per-system inertia of a batch of independent systems (batch.cu)
 void launch_system_inertia(const DevState& s, const int* node_sys, int nn, int* sys_inertia,

@@ -70,7 +70,7 @@ __device__ __forceinline__ bool is_second(const unsigned* secw, int p) {
 __global__ void __launch_bounds__(kSbThreads, 1)
     forward_big_kernel(DevPlan p, DevState s, const int* __restrict__ nodes,
                        double* __restrict__ x, int ldx, int nrhs, int r0rhs, int nr,
-                       double* __restrict__ upool) {
+                       double* __restrict__ upool, int* done, int done_value) {
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank();
   const int node = nodes[blockIdx.x / kSbCL];
@@ -284,11 +284,13 @@ __global__ void __launch_bounds__(kSbThreads, 1)
   for (int i = max(rb, npiv) + tid; i < re; i += kSbThreads)
     for (int r = 0; r < nr; r++) uo[(size_t)r * m + (i - npiv)] = v[(size_t)r * R + (i - rb)];
   cl.sync();  // partners read through DSMEM are done
+  if (rank == 0 && tid == 0) done[node] = done_value;  // for the launches that follow
 }
 
 __global__ void __launch_bounds__(kSbThreads)
     backward_big_kernel(DevPlan p, DevState s, const int* __restrict__ nodes,
-                        double* __restrict__ x, int ldx, int r0rhs, int nr) {
+                        double* __restrict__ x, int ldx, int r0rhs, int nr, int* done,
+                        int done_value) {
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank();
   const int node = nodes[blockIdx.x / kSbCL];
@@ -432,6 +434,7 @@ __global__ void __launch_bounds__(kSbThreads)
     }
   }
   cl.sync();
+  if (rank == 0 && tid == 0) done[node] = done_value;
 }
 
 size_t fwd_big_smem(int fmax) {
@@ -484,44 +487,23 @@ cudaError_t configure_solve_big_kernels() {
                               cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
 }
 
-int launch_forward_big(const DevPlan& p, const DevState& s, const int* nodes, int count,
-                       double* x, int ldx, int nrhs, double* upool, int fmax,
-                       cudaStream_t stream, cudaError_t* err) {
-  if (count <= 0) return 0;
-  int n = 0;
-  for (int r0 = 0; r0 < nrhs; r0 += kSbRhs) {
-    const int nr = (nrhs - r0 < kSbRhs) ? nrhs - r0 : kSbRhs;
-    cudaLaunchAttribute a[1];
-    cudaLaunchConfig_t cfg = cluster_cfg(count, fwd_big_smem(fmax), stream, a);
-    const cudaError_t e =
-        cudaLaunchKernelEx(&cfg, forward_big_kernel, p, s, nodes, x, ldx, nrhs, r0, nr, upool);
-    if (e != cudaSuccess) {
-      *err = e;
-      return n;
-    }
-    n++;
-  }
-  return n;
+cudaError_t launch_forward_big(const DevPlan& p, const DevState& s, const SolveSpan& sp, double* x,
+                               int ldx, int nrhs, int r0, int nr, double* upool,
+                               cudaStream_t stream) {
+  if (sp.count <= 0) return cudaSuccess;
+  cudaLaunchAttribute a[1];
+  cudaLaunchConfig_t cfg = cluster_cfg(sp.count, fwd_big_smem(sp.fmax), stream, a);
+  return cudaLaunchKernelEx(&cfg, forward_big_kernel, p, s, sp.nodes, x, ldx, nrhs, r0, nr, upool,
+                            sp.fdone, 2 * sp.epoch + 1);
 }
 
-int launch_backward_big(const DevPlan& p, const DevState& s, const int* nodes, int count,
-                        double* x, int ldx, int nrhs, int fmax, cudaStream_t stream,
-                        cudaError_t* err) {
-  if (count <= 0) return 0;
-  int n = 0;
-  for (int r0 = 0; r0 < nrhs; r0 += kSbRhs) {
-    const int nr = (nrhs - r0 < kSbRhs) ? nrhs - r0 : kSbRhs;
-    cudaLaunchAttribute a[1];
-    cudaLaunchConfig_t cfg = cluster_cfg(count, bwd_big_smem(fmax), stream, a);
-    const cudaError_t e =
-        cudaLaunchKernelEx(&cfg, backward_big_kernel, p, s, nodes, x, ldx, r0, nr);
-    if (e != cudaSuccess) {
-      *err = e;
-      return n;
-    }
-    n++;
-  }
-  return n;
+cudaError_t launch_backward_big(const DevPlan& p, const DevState& s, const SolveSpan& sp,
+                                double* x, int ldx, int r0, int nr, cudaStream_t stream) {
+  if (sp.count <= 0) return cudaSuccess;
+  cudaLaunchAttribute a[1];
+  cudaLaunchConfig_t cfg = cluster_cfg(sp.count, bwd_big_smem(sp.fmax), stream, a);
+  return cudaLaunchKernelEx(&cfg, backward_big_kernel, p, s, sp.nodes, x, ldx, r0, nr, sp.bdone,
+                            2 * sp.epoch + 1);
 }
 
 }  // namespace b200ldl
