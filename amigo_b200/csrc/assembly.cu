@@ -32,14 +32,52 @@
 
 namespace {
 
-__global__ void csr_gather_kernel(int nnz, const long long* __restrict__ ptr,
-                                  const long long* __restrict__ src,
-                                  const double* __restrict__ blocks, double* __restrict__ vals) {
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < nnz; p += gridDim.x * blockDim.x) {
-    double v = 0.0;
-    const long long e = ptr[p + 1];
-    for (long long s = ptr[p]; s < e; s++) v += blocks[src[s]];
-    vals[p] = v;
+// Contributions per CSR entry are few (1 to 4 in the mesh workloads), so an
+// entry is bound by the latency of ptr -> src -> block value and the kernel by
+// the bytes of the plan: the indices are 32-bit where the plan allows (half
+// the plan's bytes), and a thread takes kPer entries at a time, whose first
+// two contributions are loaded before any is added. An entry's sum stays in
+// order from zero. Plane-stress elements, 256 x 256 (151 MB of blocks, 6.09 M
+// entries): 69.4 us with 64-bit indices and an entry at a time, 53.1 us now (one
+// entry at a time 62, four 64).
+constexpr int kPer = 2;
+
+template <typename Index>
+__global__ void __launch_bounds__(256)
+    csr_gather_kernel(int nnz, const Index* __restrict__ ptr, const Index* __restrict__ src,
+                      const double* __restrict__ blocks, double* __restrict__ vals) {
+  const int per_cta = blockDim.x * kPer;
+  for (long long p0 = (long long)blockIdx.x * per_cta; p0 < nnz;
+       p0 += (long long)gridDim.x * per_cta) {
+    Index b[kPer], e[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; u++) {
+      const long long p = p0 + threadIdx.x + u * blockDim.x;
+      b[u] = p < nnz ? __ldg(ptr + p) : 0;
+      e[u] = p < nnz ? __ldg(ptr + p + 1) : 0;
+    }
+    Index s0[kPer], s1[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; u++) {
+      s0[u] = b[u] < e[u] ? __ldg(src + b[u]) : 0;
+      s1[u] = b[u] + 1 < e[u] ? __ldg(src + b[u] + 1) : 0;
+    }
+    double x0[kPer], x1[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; u++) {
+      x0[u] = b[u] < e[u] ? blocks[s0[u]] : 0.0;
+      x1[u] = b[u] + 1 < e[u] ? blocks[s1[u]] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < kPer; u++) {
+      const long long p = p0 + threadIdx.x + u * blockDim.x;
+      if (p >= nnz) continue;
+      double v = 0.0;
+      if (b[u] < e[u]) v += x0[u];
+      if (b[u] + 1 < e[u]) v += x1[u];
+      for (Index q = b[u] + 2; q < e[u]; q++) v += blocks[src[q]];
+      __stcs(vals + p, v);
+    }
   }
 }
 
@@ -59,7 +97,8 @@ struct b200ldl_assembly {
   long long nvals = 0;    // block values expected (sum over groups of nelem * ncomp^2)
   long long dropped = 0;  // contributions outside the pattern
   std::vector<long long> ptr, src;  // the plan, host copy
-  DevArr<long long> d_ptr, d_src;
+  DevArr<long long> d_ptr, d_src;  // for factorizations from element blocks
+  DevArr<int> d_ptr32, d_src32;    // for the gather, where the plan fits
   bool uploaded = false;
   std::string last_error;
 };
@@ -96,6 +135,17 @@ int upload(b200ldl_assembly* a) {
   if (e == cudaSuccess && !a->src.empty())
     e = cudaMemcpy(a->d_src.ptr, a->src.data(), a->src.size() * sizeof(long long),
                    cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && a->nvals <= 2147483647LL && a->src.size() <= 2147483647u) {
+    const std::vector<int> p32(a->ptr.begin(), a->ptr.end());
+    const std::vector<int> s32(a->src.begin(), a->src.end());
+    e = cudaMalloc(&a->d_ptr32.ptr, np * sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc(&a->d_src32.ptr, ns * sizeof(int));
+    if (e == cudaSuccess)
+      e = cudaMemcpy(a->d_ptr32.ptr, p32.data(), np * sizeof(int), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && !s32.empty())
+      e = cudaMemcpy(a->d_src32.ptr, s32.data(), s32.size() * sizeof(int),
+                     cudaMemcpyHostToDevice);
+  }
   if (e != cudaSuccess) return afail(a, -3, "CUDA error: %s", cudaGetErrorString(e));
   a->uploaded = true;
   return 0;
@@ -173,9 +223,14 @@ int b200ldl_assembly_values(b200ldl_assembly_t a, const double* blocks, double* 
   const int st = upload(a);
   if (st != 0) return st;
   const int threads = 256;
-  const int grid = std::max(1, std::min((a->nnz + threads - 1) / threads, 148 * 8));
-  csr_gather_kernel<<<grid, threads, 0, static_cast<cudaStream_t>(stream)>>>(
-      a->nnz, a->d_ptr.ptr, a->d_src.ptr, blocks, vals);
+  const int per_cta = threads * kPer;
+  const int grid = std::max(1, std::min((a->nnz - 1) / per_cta + 1, 148 * 64));
+  const cudaStream_t st_ = static_cast<cudaStream_t>(stream);
+  if (a->d_ptr32.ptr)
+    csr_gather_kernel<<<grid, threads, 0, st_>>>(a->nnz, a->d_ptr32.ptr, a->d_src32.ptr, blocks,
+                                                 vals);
+  else
+    csr_gather_kernel<<<grid, threads, 0, st_>>>(a->nnz, a->d_ptr.ptr, a->d_src.ptr, blocks, vals);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return afail(a, -3, "CUDA error: %s", cudaGetErrorString(e));
   return 0;
