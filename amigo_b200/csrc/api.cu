@@ -616,15 +616,23 @@ void run_factor_once(b200ldl_t h, const double* vals, const double* diag, bool m
     CK(cudaMemsetAsync(h->d_ticket.ptr, 0, sizeof(int) * std::max(1, h->num_levels), h->stream));
     for (int l = 0; l < h->num_levels; l++) {
       const int b = h->level_ptr[l];
-      // consecutive levels without big fronts share a launch: twice the
+      // Consecutive levels without big fronts share a launch: twice the
       // widest level's CTAs, so that fronts of the next level load their own
       // entries while this level's are factored, and no more than can be
-      // resident
+      // resident. A level that fills the GPU by itself only joins levels of
+      // its kernel variant (its CTAs per SM count there: 80,000 leaves of the
+      // 256 x 256 plane-stress tree with the variant of larger fronts cost
+      // 2.5 ms more than a launch saves).
+      constexpr int kFill = 148 * 4;
       int l1 = l + 1, fcap = h->level_fcap[l], width = h->level_ptr[l + 1] - b;
       if (!h->level_big[l])
         for (; l1 < h->num_levels && !h->level_big[l1]; l1++) {
+          const int w1 = h->level_ptr[l1 + 1] - h->level_ptr[l1];
+          if (std::max(width, w1) > kFill &&
+              factor_variant(fcap) != factor_variant(h->level_fcap[l1]))
+            break;
           fcap = std::max(fcap, h->level_fcap[l1]);
-          width = std::max(width, h->level_ptr[l1 + 1] - h->level_ptr[l1]);
+          width = std::max(width, w1);
         }
       const int cnt = h->level_ptr[l1] - b;
       const bool run = l1 > l + 1;
@@ -633,7 +641,7 @@ void run_factor_once(b200ldl_t h, const double* vals, const double* diag, bool m
       h->prof.begin(h->stream);
       launch_factor_level(h->plan, h->st, h->d_level_nodes.ptr + b, cnt,
                           run ? h->d_ticket.ptr + l : nullptr,
-                          run ? std::min({cnt, 2 * width, 148 * 4}) : cnt, fcap, h->level_big[l],
+                          run ? std::min({cnt, 2 * width, kFill}) : cnt, fcap, h->level_big[l],
                           prm, h->stream, vals, diag);
       h->prof.end(kPhFront, h->stream, 1);
       CK(cudaGetLastError());

@@ -48,6 +48,16 @@
 // cannot delay: the candidates its tests leave are finished by the chained
 // panels (Bunch-Kaufman) after the level's launch.
 //
+// What a panel step costs is mostly fixed: three grid barriers, one warp's
+// work on the block, and chains of global loads. So each phase loads before
+// it computes, an item's front is described in shared memory (Info), the
+// one-warp phase counts its instructions (a panel's block 79,000 -> 48,000
+// cycles), delays exchange in phase D only what the block needs (30,000 ->
+// 11,000-23,000 cycles on a one-front level), and the trailing tiles use
+// mma.m8n8k4.f64 with the next tile's loads in flight. Plane stress 256 x
+// 256, record of a neighbouring iterate: 291 -> 248 ms of panel levels a
+// factorization; hex elasticity 11^3 with a dense row: 133 -> 112 ms.
+//
 // The phases run in one cooperative launch per level, separated by grid-wide
 // barriers: three per panel step. Every CTA runs the same phases and
 // barriers; the loop ends for all of them on a count that the barrier makes
@@ -74,11 +84,12 @@ namespace b200ldl {
 namespace {
 
 constexpr int kBlk = 32;  // candidates per panel
-constexpr int kLd = kBlk + 1;
+constexpr int kLd = kBlk + 2;  // even: two entries of a row per shared-memory load
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kTileU = 64;          // trailing-update tile
 constexpr int kChunkFronts = 1024;  // fronts per work-item prefix
+constexpr unsigned long long kInfBits = 0x7ff0000000000000ull;
 
 // per-front scratch (doubles at xoff)
 constexpr int kXNext = kAppNextColmax;      // [32] next panel's column maxima below (bits)
@@ -102,7 +113,9 @@ constexpr int kIDcnt = 102;   // candidates to delay at the next step
 constexpr int kIDpos = 103;   // [32] their positions, decreasing
 constexpr int kINp = kIDpos + kBlk;  // pivots that pass the exact tests (set by phase R)
 constexpr int kIRdone = kINp + 1;    // phase-R items of the panel finished
-constexpr int kINint = kIRdone + 1;
+constexpr int kISwaps = kIRdone + 1;   // interchanges that phase R carries out
+constexpr int kISwapB = kISwaps + 1;   // candidates before them (b = that - 1 - q)
+constexpr int kINint = kISwapB + 1;
 static_assert(kXInt + (kINint + 1) / 2 <= kAppScratch, "a-posteriori scratch size");
 
 __device__ __forceinline__ double fsym(const double* F, int f, int a, int b) {
@@ -142,13 +155,25 @@ __device__ __forceinline__ double warp_max(double v) {
 // The L entries (l0, l1) of a row whose W entries are (a, b) under the 2x2
 // pivot d = (d11, d21, d22): (a, b) D^-1, with explicit fused multiply-adds so
 // that every kernel that forms them gets the same values.
-__device__ __forceinline__ void l_2x2(const double* d, double a, double b, double& l0,
-                                      double& l1) {
+__device__ __forceinline__ void inv_2x2(const double* d, double* inv) {
   const double d11 = d[0], d21 = d[1], d22 = d[2];
   const double di = 1.0 / (d11 * d22 - d21 * d21);
-  const double i00 = d22 * di, i01 = -d21 * di, i11 = d11 * di;
-  l0 = fma(a, i00, b * i01);
-  l1 = fma(a, i01, b * i11);
+  inv[0] = d22 * di;
+  inv[1] = -d21 * di;
+  inv[2] = d11 * di;
+}
+__device__ __forceinline__ double l_first(const double* inv, double a, double b) {
+  return fma(a, inv[0], __dmul_rn(b, inv[1]));
+}
+__device__ __forceinline__ double l_second(const double* inv, double a, double b) {
+  return fma(a, inv[1], __dmul_rn(b, inv[2]));
+}
+__device__ __forceinline__ void l_2x2(const double* d, double a, double b, double& l0,
+                                      double& l1) {
+  double inv[3];
+  inv_2x2(d, inv);
+  l0 = l_first(inv, a, b);
+  l1 = l_second(inv, a, b);
 }
 
 // ------------------------------------------------------------- shared memory
@@ -156,32 +181,33 @@ __device__ __forceinline__ void l_2x2(const double* d, double a, double b, doubl
 struct WarpDiag {  // phase D, one per warp
   double A[kBlk][kLd];  // the block, symmetric, factored in place
   double Lb[kBlk][kLd];
-  double dd[3 * kBlk], cin[kBlk], rin[kBlk], below0[kBlk];
-  int perm[kBlk], kind[kBlk], dlt[kBlk];
+  double below0[kBlk];
+  int perm[kBlk], dlt[kBlk];
   int var[kBlk], part[kBlk];  // block candidates' variables and recorded 2x2 partners
 };
 
 struct RowsSm {  // phases R and A
-  double Ls[kBlk][kLd];
+  alignas(16) double Ls[kBlk][kLd];
   double red[kWarps][kBlk];
   double sd[3 * kBlk], sinv[kBlk];
+  double inv[kBlk][3];  // phase A: inverses of the 2x2 pivots
   double scm[kBlk], srm[kBlk];  // phase A: column maxima over the front, 2x2 partner's block part
   int sperm[kBlk], skind[kBlk];
   int np;
 };
 
 // The reference's tests for the accepted pivots of a panel, with the column
-// maxima over the whole front (staged in shared memory by phase A): number
-// of leading pivots that pass.
+// maxima over the whole front (staged in shared memory), by one warp, a lane
+// per pivot: number of leading pivots that pass.
 __device__ int passing_prefix(const RowsSm& sm, int acc, double ustab, double tol) {
-  int p = 0;
-  while (p < acc) {
+  const int p = threadIdx.x & 31;
+  bool ok = true;
+  if (p < acc) {
     const double cm = sm.scm[p];
     if (sm.skind[p] == 1) {
       const double d = sm.sd[3 * p];
-      if (!(fabs(d) >= tol && fabs(d) >= ustab * cm)) break;
-      p += 1;
-    } else {
+      ok = fabs(d) >= tol && fabs(d) >= ustab * cm;
+    } else if (sm.skind[p] == 2) {
       const double d11 = sm.sd[3 * p], d21 = sm.sd[3 * p + 1], d22 = sm.sd[3 * p + 2];
       const double det = fabs(d11 * d22 - d21 * d21);
       const double ad21 = fabs(d21);
@@ -189,17 +215,20 @@ __device__ int passing_prefix(const RowsSm& sm, int acc, double ustab, double to
       // the partner's maximum: its block part (srm) and its maximum below
       // (scm of the second position, whose block part phase D leaves at 0)
       const double rm = fmax(sm.srm[p], sm.scm[p + 1]);
-      if (!(det >= tol && delta >= ustab * cm && delta >= ustab * rm)) break;
-      p += 2;
+      ok = det >= tol && delta >= ustab * cm && delta >= ustab * rm;
     }
   }
-  return p;
+  const unsigned bad = __ballot_sync(0xffffffffu, !ok);
+  return bad ? __ffs(bad) - 1 : acc;
 }
 
+// row stride of the panels in shared memory: the four pivots that a warp's
+// lanes read at once start 8 banks apart
+constexpr int kTileLdU = kTileU + 4;
 struct UpdSm {  // phase U
-  double As[kBigPanelMax][kTileU];
-  double Bs[kBigPanelMax][kTileU];
-  double ud[3 * kBlk], usinv[kBlk];  // the panel's D, when L is formed from W
+  double As[kBigPanelMax][kTileLdU];
+  double Bs[kBigPanelMax][kTileLdU];
+  double ud[3 * kBlk], usinv[kBlk];  // the panel's D^-1, when L is formed from W
   int ukind[kBlk];
 };
 
@@ -208,50 +237,58 @@ struct Prefix {  // work items of up to kChunkFronts fronts
   long long wsum[kWarps];
 };
 
+// What a work item needs of its front, gathered by front_prefix so that an
+// item does not start with a chain of global loads.
+struct Info {
+  double *F, *W, *X;
+  int f, k, nbk, np;  // np: pivots accepted in the block (phase R) or passing
+  int rows;           // row chunks (phases R and A); 0: not in this step
+  int moved;
+  int swaps, swap_b;  // interchanges left to phase R
+};
+
 constexpr size_t cmax(size_t a, size_t b) { return a > b ? a : b; }
 // the mixed-precision tile places the tensor-core operands after the FP64
 // tiles' panels, 1 KB aligned
 constexpr size_t kOpsOffset = (sizeof(UpdSm) + 1023) / 1024 * 1024;
+// the work items' fronts come first, then what the phase uses
+constexpr size_t kInfoBytes = (sizeof(Info) * kChunkFronts + 1023) / 1024 * 1024;
 constexpr size_t kDynSmem =
-    cmax(sizeof(WarpDiag) * kWarps,
-         cmax(sizeof(RowsSm), kOpsOffset + umma::kSmemFloats * sizeof(float)));
+    kInfoBytes + cmax(sizeof(WarpDiag) * kWarps,
+                      cmax(sizeof(RowsSm), kOpsOffset + umma::kSmemFloats * sizeof(float)));
 
 // Exclusive prefix of cnt(i) over i in [0, nl) into P.ptr (CTA-wide; nl <=
-// kChunkFronts). Returns the total.
+// kChunkFronts). Returns the total. A thread counts one front per round, so
+// that the chains of loads of cnt run side by side.
 template <typename Count>
 __device__ long long front_prefix(Prefix& P, int nl, Count cnt) {
-  constexpr int per = kChunkFronts / kThreads;
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int w = tid >> 5;
-  long long c[per];
-  long long mine = 0;
-#pragma unroll
-  for (int u = 0; u < per; u++) {
-    const int i = tid * per + u;
-    c[u] = (i < nl) ? cnt(i) : 0;
-    mine += c[u];
-  }
-  long long incl = mine;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const long long v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += v;
-  }
-  if (lane == 31) P.wsum[w] = incl;
-  __syncthreads();
   long long base = 0;
-  for (int q = 0; q < w; q++) base += P.wsum[q];
-  long long run = base + incl - mine;
   if (tid == 0) P.ptr[0] = 0;
+  for (int i0 = 0; i0 < nl; i0 += kThreads) {
+    const int i = i0 + tid;
+    long long incl = (i < nl) ? cnt(i) : 0;
 #pragma unroll
-  for (int u = 0; u < per; u++) {
-    run += c[u];
-    const int i = tid * per + u;
-    if (i < nl) P.ptr[i + 1] = run;
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (lane == 31) P.wsum[w] = incl;
+    __syncthreads();
+    long long before = base, all = base;
+#pragma unroll
+    for (int q = 0; q < kWarps; q++) {
+      const long long v = P.wsum[q];
+      if (q < w) before += v;
+      all += v;
+    }
+    if (i < nl) P.ptr[i + 1] = before + incl;
+    base = all;
+    __syncthreads();
   }
-  __syncthreads();
-  return P.ptr[nl];
+  return base;
 }
 
 // front of work item t: the last i with ptr[i] <= t
@@ -298,7 +335,8 @@ __device__ __forceinline__ void group_sync() {
 // CTAs); g is the thread's index in the group. Returns 1 if the front takes
 // part in this step.
 template <int NT>
-__device__ int phase_d_prepare(const DevState& s, BigFront* B, int* done, int* meta, int g) {
+__device__ int phase_d_prepare(const DevState& s, BigFront* B, int* done, int* meta, int g,
+                               WarpDiag& w) {
   const int f = B->f;
   double* F = s.dpool + B->doff;
   double* X = s.dpool + B->xoff;
@@ -318,12 +356,30 @@ __device__ int phase_d_prepare(const DevState& s, BigFront* B, int* done, int* m
     if (B->state == 1) finish_front(s, B, done, meta);
   }
   group_sync<NT>();
+  int swaps = 0;
   if (B->pending > 0 && B->state == 0) {
-    // the candidates to delay move behind the remaining candidates, largest
-    // position first so that no interchange moves another one still to go
+    // The candidates to delay move behind the remaining candidates, largest
+    // position first so that no interchange moves another one still to go.
+    // Only the entries between the next block's rows and the rows behind the
+    // candidates are exchanged here (what the block and the maxima need):
+    // one CTA would take 15,000 cycles and more for a 3,600-row front's rows,
+    // an 8-byte access per column, so every other row is left to phase R,
+    // whose items own the rows. A front that is done with its candidates has
+    // no phase R: all its rows are exchanged at once.
     const int nd = xi[kIDcnt];
     const int k = B->k;
-    int ncand = B->ncand;
+    const int n0 = B->ncand;
+    const int n1 = n0 - nd;
+    const bool all = k >= n1;
+    const int blk1 = min(k + kBlk, f);  // rows of the block
+    const int far = max(n1, blk1);      // and of [n1, n0) beyond it
+    const int near = blk1 - k;
+    const int few = near + max(0, n0 - far);
+    if (!all && g < kBlk) {
+      // what stands at the block's positions, and at [n1, n0)
+      w.perm[g] = k + g;
+      w.part[g] = n0 - 1 - g;
+    }
     // The next panel's first test needs the exact maximum below the block
     // (rows from k + kBlk on) of every block column. An interchange of rows
     // a (in the block) and b (below it) takes row b's entry out of a
@@ -334,9 +390,10 @@ __device__ int phase_d_prepare(const DevState& s, BigFront* B, int* done, int* m
     const bool trk = g < kBlk && ct < f;
     bool stale = false;
     double mx = trk ? X[kXNext + g] : 0.0;
+    group_sync<NT>();
     for (int q = 0; q < nd; q++) {
       const int a = xi[kIDpos + q];
-      const int b = ncand - 1;
+      const int b = n0 - 1 - q;
       if (a < b) {
         if (trk) {
           if (ct == a || ct == b) {
@@ -351,16 +408,18 @@ __device__ int phase_d_prepare(const DevState& s, BigFront* B, int* done, int* m
         // the pairs of a symmetric interchange are distinct entries: eight
         // passes of the group load theirs before any is stored back
         constexpr int kU = 8;
-        for (int j0 = 0; j0 < f; j0 += NT * kU) {
+        const int nj = all ? f : few;
+        for (int j0 = 0; j0 < nj; j0 += NT * kU) {
           double* p[kU];
           double* r[kU];
           double vp[kU], vr[kU];
 #pragma unroll
           for (int u = 0; u < kU; u++) {
-            const int j = j0 + NT * u + g;
+            const int jj = j0 + NT * u + g;
             p[u] = nullptr;
             r[u] = nullptr;
-            if (j >= f || j == b) continue;
+            const int j = all ? jj : jj < near ? k + jj : far + jj - near;
+            if (jj >= nj || j == b) continue;
             if (j < a) {
               p[u] = F + a + (size_t)f * j;
               r[u] = F + b + (size_t)f * j;
@@ -395,9 +454,15 @@ __device__ int phase_d_prepare(const DevState& s, BigFront* B, int* done, int* m
           t = orig[a];
           orig[a] = orig[b];
           orig[b] = t;
+          if (!all) {
+            int* pa = w.perm + (a - k);
+            int* pb = b < blk1 ? w.perm + (b - k) : w.part + q;
+            t = *pa;
+            *pa = *pb;
+            *pb = t;
+          }
         }
       }
-      ncand--;
       group_sync<NT>();
     }
     // the block columns whose maximum below may have changed, formed again
@@ -414,23 +479,44 @@ __device__ int phase_d_prepare(const DevState& s, BigFront* B, int* done, int* m
       redo = redo_sh;
     }
     if (trk && !stale) X[kXNext + g] = mx;
-    const int lane = g & 31, wq = g >> 5;
-    for (int i = wq; i < kBlk; i += NT / 32) {
-      if (!((redo >> i) & 1u)) continue;
-      const double* col = F + (size_t)f * (k + i);
-      double m = 0.0;
-      for (int r = k + kBlk + lane; r < f; r += 32) m = fmax(m, fabs(col[r]));
-      m = warp_max(m);
-      if (lane == 0) X[kXNext + i] = m;
+    const int lane = g & 31;
+    // a column is read by the whole group, eight entries of a thread in
+    // flight; non-negative doubles order as their bits
+    for (unsigned left = all ? 0u : redo; left; left &= left - 1) {
+      const int i = __ffs(left) - 1;
+      if (g == 0) X[kXNext + i] = 0.0;
+      group_sync<NT>();
+      // rows not yet exchanged have the column where it stood
+      const int was = w.perm[i];
+      unsigned long long m = 0;
+      for (int r0 = k + kBlk; r0 < f; r0 += 8 * NT) {
+        unsigned long long e[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+          const int r = r0 + NT * u + g;
+          const int c = (r >= n1 && r < n0) ? k + i : was;
+          e[u] = r < f ? (unsigned long long)__double_as_longlong(fabs(fsym(F, f, r, c))) : 0ull;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+          if (e[u] <= kInfBits && e[u] > m) m = e[u];  // NaN entries do not take part
+      }
+      const double wm = warp_max(__longlong_as_double((long long)m));
+      if (lane == 0 && wm > 0.0)
+        atomicMax(reinterpret_cast<unsigned long long*>(X + kXNext) + i,
+                  (unsigned long long)__double_as_longlong(wm));
     }
     group_sync<NT>();
     if (g == 0) {
-      B->ncand = ncand;
+      B->ncand = n1;
       B->pending = 0;
-      if (B->k >= ncand) finish_front(s, B, done, meta);
+      xi[kISwapB] = n0;
+      if (all) finish_front(s, B, done, meta);
     }
+    swaps = all ? 0 : nd;
     group_sync<NT>();
   }
+  if (g == 0) xi[kISwaps] = swaps;
   return B->state == 0 ? 1 : 0;
 }
 
@@ -449,6 +535,8 @@ __device__ int phase_d_block(const DevState& s, const FactorParams& prm, BigFron
   const int k = B->k;
   const int ncand = B->ncand;
   const int nbk = max(0, min(kBlk, ncand - k));
+  bool finite;     // every entry of the block is finite
+  unsigned hints;  // positions whose candidate was in a 2x2 with the next one
   {
     // the block's lower triangle, one coalesced column per load (all loads
     // in flight before the shared-memory stores), mirrored above
@@ -470,15 +558,22 @@ __device__ int phase_d_block(const DevState& s, const FactorParams& prm, BigFron
     }
     w.var[lane] = var;
     w.part[lane] = part;
+    int top = 0;
+#pragma unroll
+    for (int j = 0; j < kBlk; j++) top = max(top, __double2hiint(v[j]) & 0x7fffffff);
+    finite = __all_sync(0xffffffffu, top < 0x7ff00000);
+    const int vnext = __shfl_down_sync(0xffffffffu, var, 1);
+    hints = __ballot_sync(0xffffffffu, lane < 31 && var >= 0 && vnext >= 0 && part == vnext);
   }
   w.perm[lane] = lane;
-  w.kind[lane] = 0;
   w.dlt[lane] = -1;
-  w.cin[lane] = 0.0;
-  w.rin[lane] = 0.0;
-  w.dd[3 * lane] = w.dd[3 * lane + 1] = w.dd[3 * lane + 2] = 0.0;
-  w.below0[lane] = __longlong_as_double(
-      (long long)reinterpret_cast<unsigned long long*>(X + kXNext)[lane]);
+  // of the pivot at position `lane`: its kind, D, and the block's part of its
+  // column maximum and of its 2x2 partner's (left at 0 for a 1x1 that passed
+  // where it stood: it passed against those entries already)
+  int kind = 0;
+  double dd0 = 0.0, dd1 = 0.0, dd2 = 0.0, cin = 0.0, rin = 0.0;
+  // (partly the result of atomics: read from L2)
+  w.below0[lane] = __ldcg(X + kXNext + lane);
   // read: the trailing update of this panel fills them again for the next
   X[kXNext + lane] = 0.0;
   __syncwarp();
@@ -499,18 +594,63 @@ __device__ int phase_d_block(const DevState& s, const FactorParams& prm, BigFron
   // (i, j) minus L(max(i, j), q) W(min(i, j), q) for each earlier pivot q in
   // order, the products and the order of the reference's lower-triangle
   // update. Lane i forms row i.
+  // One warp runs this alone, so what counts is its number of instructions:
+  // two entries of a row per load, eight pivots' products at a time, and no
+  // test of q against t: beyond t the L entries are still zero, and zero
+  // times a finite entry as loaded leaves the sum as it is (a block with an
+  // infinity or NaN goes pivot by pivot).
   auto form = [&](int j) -> double {
-    if (lane < t || lane >= nbk) return 0.0;
     const int hi = max(lane, j), lo = min(lane, j);
     double v = w.A[lane][j];
-    for (int q = 0; q < t; q++) v = fma(-w.Lb[hi][q], w.A[lo][q], v);
-    return v;
+    if (finite) {
+      const double2* lr = reinterpret_cast<const double2*>(w.Lb[hi]);
+      const double2* wr = reinterpret_cast<const double2*>(w.A[lo]);
+      for (int q0 = 0; q0 < t; q0 += 8) {
+        double2 a[4], b[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          a[q] = lr[q0 / 2 + q];
+          b[q] = wr[q0 / 2 + q];
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          v = fma(-a[q].x, b[q].x, v);
+          v = fma(-a[q].y, b[q].y, v);
+        }
+      }
+    } else {
+      for (int q = 0; q < t; q++) v = fma(-w.Lb[hi][q], w.A[lo][q], v);
+    }
+    return (lane >= t && lane < nbk) ? v : 0.0;
   };
   while (t < nr) {
     const bool has = t + 1 < nr;
+    const bool hinted = has && ((hints >> t) & 1u);
     const double ct = form(t);  // the candidate's column
+    double c2 = 0.0;            // and its recorded partner's, or imax's
+    if (hinted) c2 = form(t + 1);
     const double wkk = __shfl_sync(kFull, ct, t);
     const double at = fabs(ct);
+    if (!hinted) {
+      // the common pivot, a 1x1 that passes where it stands: every lane tests
+      // its entry (rounded products are monotone, so that is the test against
+      // the largest one), while the reciprocal is formed
+      const double rd = 1.0 / wkk;
+      bool ok = fabs(wkk) >= tol;
+      if (lane > t && lane < nbk) ok = ok && fabs(wkk) >= u * at;
+      if (t == 0) ok = ok && fabs(wkk) >= u * w.below0[w.perm[0]];
+      if (__all_sync(kFull, ok)) {
+        if (lane >= t && lane < nbk) w.A[lane][t] = ct;
+        if (lane > t && lane < nbk) w.Lb[lane][t] = ct * rd;
+        if (lane == t) {
+          kind = 1;
+          dd0 = wkk;
+        }
+        __syncwarp();
+        t++;
+        continue;
+      }
+    }
     double bv;
     int bi;
     warp_argmax(lane > t && lane < nr, at, bv, bi);
@@ -522,18 +662,11 @@ __device__ int phase_d_block(const DevState& s, const FactorParams& prm, BigFron
     const double colmax = fmax(col_in, t == 0 ? w.below0[w.perm[t]] : 0.0);
     int stp = 0, kpiv = t;
     double row_in = 0.0;
-    double c2 = 0.0;  // the column of the partner or of imax, when formed
     // a pair that formed a 2x2 pivot in the pivot record is tried as that
     // 2x2 first (the Duff test), since a 1x1 test that sees only the block's
     // rows would accept the first of them alone and the a-posteriori test
     // would then reject it
-    bool hinted = false;
-    if (has) {
-      const int pt = w.perm[t], vn = w.var[w.perm[t + 1]];
-      hinted = w.var[pt] >= 0 && vn >= 0 && w.part[pt] == vn;
-    }
     if (hinted) {
-      c2 = form(t + 1);
       const double r2 = warp_max((lane >= t && lane < nbk && lane != t + 1) ? fabs(c2) : 0.0);
       const double rm2 = fmax(r2, t == 0 ? w.below0[w.perm[t + 1]] : 0.0);
       const double w21 = __shfl_sync(kFull, ct, t + 1), w22 = __shfl_sync(kFull, c2, t + 1);
@@ -598,6 +731,9 @@ __device__ int phase_d_block(const DevState& s, const FactorParams& prm, BigFron
         w.dlt[kdst] = q;
       }
       __syncwarp();
+      const int pl = w.perm[lane];
+      const int vn = lane < 31 ? w.var[w.perm[lane + 1]] : -1;
+      hints = __ballot_sync(kFull, w.var[pl] >= 0 && vn >= 0 && w.part[pl] == vn);
     }
     if (stp == 0) {
       if (lane == 0) w.dlt[nr - 1] = t;
@@ -618,10 +754,10 @@ __device__ int phase_d_block(const DevState& s, const FactorParams& prm, BigFron
       const double d = __shfl_sync(kFull, p1, t);
       const double li = p1 * (1.0 / d);
       if (lane > t && lane < nbk) w.Lb[lane][t] = li;
-      if (lane == 0) {
-        w.kind[t] = 1;
-        w.dd[3 * t] = d;
-        w.cin[t] = (kpiv == t) ? col_in : row_in;
+      if (lane == t) {
+        kind = 1;
+        dd0 = d;
+        cin = (kpiv == t) ? col_in : row_in;
       }
     } else {
       const double d11 = __shfl_sync(kFull, p1, t), d21 = __shfl_sync(kFull, p1, t + 1),
@@ -634,15 +770,15 @@ __device__ int phase_d_block(const DevState& s, const FactorParams& prm, BigFron
         w.Lb[lane][t] = l0;
         w.Lb[lane][t + 1] = l1;
       }
-      if (lane == 0) {
-        w.kind[t] = 2;
-        w.kind[t + 1] = 3;
-        w.dd[3 * t] = d11;
-        w.dd[3 * t + 1] = d21;
-        w.dd[3 * t + 2] = d22;
-        w.cin[t] = col_in;
-        w.rin[t] = row_in;
+      if (lane == t) {
+        kind = 2;
+        dd0 = d11;
+        dd1 = d21;
+        dd2 = d22;
+        cin = col_in;
+        rin = row_in;
       }
+      if (lane == t + 1) kind = 3;
     }
     __syncwarp();
     t += stp;
@@ -651,15 +787,16 @@ __device__ int phase_d_block(const DevState& s, const FactorParams& prm, BigFron
   const bool moved = __ballot_sync(0xffffffffu, lane < nbk && w.perm[lane] != lane) != 0u;
 
   // panel state for phases R and A
+#pragma unroll 8
   for (int q = lane; q < kBlk * kLd; q += 32) X[kXL + q] = (&w.Lb[0][0])[q];
-  X[kXD + 3 * lane] = w.dd[3 * lane];
-  X[kXD + 3 * lane + 1] = w.dd[3 * lane + 1];
-  X[kXD + 3 * lane + 2] = w.dd[3 * lane + 2];
-  X[kXCin + lane] = w.cin[lane];
-  X[kXRin + lane] = w.rin[lane];
+  X[kXD + 3 * lane] = dd0;
+  X[kXD + 3 * lane + 1] = dd1;
+  X[kXD + 3 * lane + 2] = dd2;
+  X[kXCin + lane] = cin;
+  X[kXRin + lane] = rin;
   X[kXBelow + lane] = 0.0;
   xi[kIPerm + lane] = w.perm[lane];
-  xi[kIKind + lane] = w.kind[lane];
+  xi[kIKind + lane] = kind;
   xi[kIDlt + lane] = w.dlt[lane];
   if (lane == 0) {
     xi[kIRdone] = 0;
@@ -671,10 +808,8 @@ __device__ int phase_d_block(const DevState& s, const FactorParams& prm, BigFron
     xi[kIMoved] = moved ? 1 : 0;
   }
   // the W values of the block rows for the trailing update
-  for (int q = lane; q < kBlk * kBlk; q += 32) {
-    const int i = q % kBlk, p = q / kBlk;
-    if (p < acc && i > p && i < nbk) Wg[(size_t)p * f + k + i] = w.A[i][p];
-  }
+  for (int p = 0; p < acc; p++)
+    if (lane > p && lane < nbk) Wg[(size_t)p * f + k + lane] = w.A[lane][p];
   if (moved) {
     // the block itself and the variables follow the interchanges (the factor
     // rows of earlier panels move in phase R): lane i gathers its row
@@ -704,74 +839,156 @@ __device__ __forceinline__ bool active(const DevState& s, const BigFront& B, int
   return xint(s.dpool + B.xoff)[kIStep] == step;
 }
 
-// row chunks of an active front in phases R and A (at least one, which also
-// carries the moves of earlier factor rows)
-__device__ __forceinline__ int row_chunks(const DevState& s, const BigFront& B, int step) {
-  if (!active(s, B, step)) return 0;
-  const int* xi = xint(s.dpool + B.xoff);
-  const int rows = B.f - (xi[kIK] + xi[kINbk]);
-  return max(1, (rows + kThreads - 1) / kThreads);
+// The part of a front's Info that does not change during the launch.
+__device__ __forceinline__ void front_place(const DevState& s, const BigFront& B, Info& o) {
+  o.F = s.dpool + B.doff;
+  o.W = s.dpool + B.woff;
+  o.X = s.dpool + B.xoff;
+  o.f = B.f;
 }
 
-__device__ void phase_r_item(const DevState& s, const FactorParams& prm, const BigFront& B,
-                             int chunk, int nchunk, RowsSm& sm) {
+// The rest for this step: row chunks of the front, 0 if it takes no part.
+__device__ __forceinline__ int front_step(int step, Info& o) {
+  const int* xi = xint(o.X);
+  const int st = xi[kIStep], k = xi[kIK], nbk = xi[kINbk], acc = xi[kIAcc];
+  const int moved = xi[kIMoved], swaps = xi[kISwaps], swap_b = xi[kISwapB];
+  o.k = k;
+  o.nbk = nbk;
+  o.np = acc;
+  o.moved = moved;
+  o.swaps = swaps;
+  o.swap_b = swap_b;
+  o.rows = st == step ? max(1, (o.f - (k + nbk) + kThreads - 1) / kThreads) : 0;
+  return o.rows;
+}
+
+__device__ void phase_r_item(const FactorParams& prm, const Info& o, int chunk, RowsSm& sm) {
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int warp = tid >> 5;
-  double* X = s.dpool + B.xoff;
+  double* X = o.X;
   int* xi = xint(X);
-  const int f = B.f;
-  const int k = xi[kIK];
-  const int nbk = xi[kINbk];
-  const int acc = xi[kIAcc];
-  const int moved = xi[kIMoved];
-  for (int t = tid; t < kBlk * kLd; t += kThreads) (&sm.Ls[0][0])[t] = X[kXL + t];
-  if (tid < kBlk) sm.sperm[tid] = xi[kIPerm + tid];
-  __syncthreads();
-  double* F = s.dpool + B.doff;
-  double* Wg = s.dpool + B.woff;
-  if (moved) {
-    // the block's rows in the factor columns of earlier panels: one warp per
-    // column, lane i moves row k + perm[i] to row k + i
-    const bool mv = lane < nbk && sm.sperm[lane] != lane;
-    for (int j = chunk * kWarps + warp; j < k; j += nchunk * kWarps) {
-      const double v = mv ? F[(k + sm.sperm[lane]) + (size_t)f * j] : 0.0;
-      __syncwarp();
-      if (mv) F[(k + lane) + (size_t)f * j] = v;
+  const int f = o.f;
+  const int k = o.k;
+  const int nbk = o.nbk;
+  const int acc = o.np;
+  const int nchunk = o.rows;
+  double* F = o.F;
+  double* Wg = o.W;
+  const int r = k + nbk + chunk * kThreads + tid;
+  {
+    // the block's L, and where the block's rows come from
+    constexpr int kPer = (kBlk * kLd + kThreads - 1) / kThreads;
+    double t[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; u++) {
+      const int q = tid + kThreads * u;
+      t[u] = q < kBlk * kLd ? X[kXL + q] : 0.0;
+    }
+    if (tid < kBlk) sm.sperm[tid] = xi[kIPerm + tid];
+    // transposed: phase R takes L column by column, two entries per load
+#pragma unroll
+    for (int u = 0; u < kPer; u++) {
+      const int q = tid + kThreads * u;
+      if (q < kBlk * kLd && q % kLd < kBlk) sm.Ls[q % kLd][q / kLd] = t[u];
     }
   }
-  double cm[kBlk];
+  // the delays' interchanges on the rows that phase D left: this thread's
+  // row, and the warp's share of the earlier panels' factor columns
+  if (o.swaps > 0) {
+    const int* dpos = xi + kIDpos;
+    if (r >= k + kBlk && r < f && (r < o.swap_b - o.swaps || r >= o.swap_b)) {
+      for (int q = 0; q < o.swaps; q++) {
+        const int x = dpos[q], y = o.swap_b - 1 - q;
+        if (x >= y) continue;
+        double* p = F + r + (size_t)f * x;
+        double* z = r > y ? F + r + (size_t)f * y : F + y + (size_t)f * r;
+        const double vp = *p, vz = *z;
+        *p = vz;
+        *z = vp;
+      }
+    }
+    for (int j = (chunk * kWarps + warp) + lane * nchunk * kWarps; j < k;
+         j += 32 * nchunk * kWarps) {
+      for (int q = 0; q < o.swaps; q++) {
+        const int x = dpos[q], y = o.swap_b - 1 - q;
+        if (x >= y) continue;
+        double* p = F + x + (size_t)f * j;
+        double* z = F + y + (size_t)f * j;
+        const double vp = *p, vz = *z;
+        *p = vz;
+        *z = vp;
+      }
+    }
+  }
+  __syncthreads();
+  double a[kBlk];
 #pragma unroll
-  for (int p = 0; p < kBlk; p++) cm[p] = 0.0;
-  const int r = k + nbk + chunk * kThreads + tid;
-  if (r < f) {
-    double a[kBlk];
+  for (int j = 0; j < kBlk; j++)
+    a[j] = (r < f && j < nbk) ? F[r + (size_t)f * (k + sm.sperm[j])] : 0.0;
+  if (o.moved) {
+    // the block's rows in the factor columns of earlier panels: a warp takes
+    // eight columns at a time, lane i moves row k + perm[i] to row k + i
+    const bool mv = lane < nbk && sm.sperm[lane] != lane;
+    const int from = mv ? k + sm.sperm[lane] : 0;
+    for (int j0 = chunk * kWarps + warp; j0 < k; j0 += 8 * nchunk * kWarps) {
+      double t[8];
 #pragma unroll
-    for (int j = 0; j < kBlk; j++) a[j] = (j < nbk) ? F[r + (size_t)f * (k + sm.sperm[j])] : 0.0;
-    if (moved) {
+      for (int u = 0; u < 8; u++) {
+        const int j = j0 + u * nchunk * kWarps;
+        t[u] = (mv && j < k) ? F[from + (size_t)f * j] : 0.0;
+      }
+      __syncwarp();
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const int j = j0 + u * nchunk * kWarps;
+        if (mv && j < k) F[(k + lane) + (size_t)f * j] = t[u];
+      }
+    }
+    if (r < f) {
 #pragma unroll
       for (int j = 0; j < kBlk; j++)
         if (j < nbk) F[r + (size_t)f * (k + j)] = a[j];
     }
-    // W = F21 L11^-T: forward substitution with the block's unit lower L
+  }
+  // W = F21 L11^-T: forward substitution with the block's unit lower L,
+  // column by column (the later entries' chains run side by side)
 #pragma unroll
-    for (int p = 0; p < kBlk; p++) {
-      if (p < acc) {
-        double wv = a[p];
+  for (int q = 0; q < kBlk; q++) {
+    if (q < acc) {
+      if (r < f) Wg[(size_t)q * f + r] = a[q];
+      const double2* l = reinterpret_cast<const double2*>(sm.Ls[q]);
 #pragma unroll
-        for (int q = 0; q < p; q++) wv = fma(-a[q], sm.Ls[p][q], wv);
-        a[p] = wv;
-        Wg[(size_t)p * f + r] = wv;
-        cm[p] = fabs(wv);
+      for (int p2 = (q + 1) / 2; p2 < kBlk / 2; p2++) {
+        const double2 lp = l[p2];
+        if (2 * p2 > q) a[2 * p2] = fma(-a[q], lp.x, a[2 * p2]);
+        a[2 * p2 + 1] = fma(-a[q], lp.y, a[2 * p2 + 1]);
       }
     }
   }
-  // column maxima: warp, CTA, then the front (non-negative doubles compare
-  // as their bit patterns)
+  // Column maxima (non-negative doubles order as their bits; NaN entries do
+  // not take part): with every halving of the warp a lane keeps half of the
+  // columns, then the CTA's and the front's maxima.
+  {
+    unsigned long long m[kBlk];
 #pragma unroll
-  for (int p = 0; p < kBlk; p++) {
-    const double v = warp_max(cm[p]);
-    if (lane == 0) sm.red[warp][p] = v;
+    for (int p = 0; p < kBlk; p++) {
+      const unsigned long long e =
+          (unsigned long long)__double_as_longlong(a[p]) & 0x7fffffffffffffffull;
+      m[p] = (p < acc && r < f && e <= kInfBits) ? e : 0ull;
+    }
+#pragma unroll
+    for (int n = kBlk / 2; n >= 1; n >>= 1) {
+      const bool up = lane & n;
+#pragma unroll
+      for (int i = 0; i < n; i++) {
+        const unsigned long long keep = up ? m[i + n] : m[i];
+        const unsigned long long send = up ? m[i] : m[i + n];
+        const unsigned long long got = __shfl_xor_sync(0xffffffffu, send, n);
+        m[i] = keep > got ? keep : got;
+      }
+    }
+    sm.red[warp][lane] = __longlong_as_double((long long)m[0]);  // column `lane`
   }
   __syncthreads();
   if (tid < acc) {
@@ -799,9 +1016,10 @@ __device__ void phase_r_item(const DevState& s, const FactorParams& prm, const B
           *(reinterpret_cast<volatile unsigned long long*>(X + kXBelow) + tid);
       sm.scm[tid] = fmax(X[kXCin + tid], __longlong_as_double((long long)bl));
       sm.srm[tid] = X[kXRin + tid];
+      __syncwarp();
+      const int np = passing_prefix(sm, acc, prm.ustab, prm.pivot_tol);
+      if (tid == 0) xi[kINp] = np;
     }
-    __syncthreads();
-    if (tid == 0) xi[kINp] = passing_prefix(sm, acc, prm.ustab, prm.pivot_tol);
   }
   __syncthreads();
 }
@@ -809,40 +1027,48 @@ __device__ void phase_r_item(const DevState& s, const FactorParams& prm, const B
 // ---------------------------------------------------------------- phase A
 
 
-__device__ void phase_a_item(const DevState& s, const FactorParams& prm, BigFront* B, int chunk,
+__device__ void phase_a_item(const DevState& s, BigFront* B, const Info& o, int chunk,
                              RowsSm& sm) {
   const int tid = threadIdx.x;
-  double* X = s.dpool + B->xoff;
+  double* X = o.X;
   int* xi = xint(X);
-  const int f = B->f;
-  const int k = xi[kIK];
-  const int nbk = xi[kINbk];
-  for (int t = tid; t < kBlk * kLd; t += kThreads) (&sm.Ls[0][0])[t] = X[kXL + t];
+  const int f = o.f;
+  const int k = o.k;
+  const int nbk = o.nbk;
+  const int np = o.np;
+  double* F = o.F;
+  const double* Wg = o.W;
+  const int r = k + nbk + chunk * kThreads + tid;
+  // the row's W entries, all loads in flight
+  double w[kBlk];
+#pragma unroll
+  for (int p = 0; p < kBlk; p++) w[p] = (r < f && p < np) ? Wg[(size_t)p * f + r] : 0.0;
+  if (chunk == 0)
+    for (int t = tid; t < kBlk * kLd; t += kThreads) (&sm.Ls[0][0])[t] = X[kXL + t];
   if (tid < kBlk) {
-    sm.skind[tid] = xi[kIKind + tid];
-    sm.sd[3 * tid] = X[kXD + 3 * tid];
-    sm.sd[3 * tid + 1] = X[kXD + 3 * tid + 1];
-    sm.sd[3 * tid + 2] = X[kXD + 3 * tid + 2];
+    const int kd = xi[kIKind + tid];
+    const double d[3] = {X[kXD + 3 * tid], X[kXD + 3 * tid + 1], X[kXD + 3 * tid + 2]};
+    sm.skind[tid] = kd;
+    sm.sd[3 * tid] = d[0];
+    sm.sd[3 * tid + 1] = d[1];
+    sm.sd[3 * tid + 2] = d[2];
     // 1x1 pivots scale their column by 1/d, as the reference does
-    sm.sinv[tid] = (xi[kIKind + tid] == 1) ? 1.0 / X[kXD + 3 * tid] : 0.0;
+    sm.sinv[tid] = (kd == 1) ? 1.0 / d[0] : 0.0;
+    if (kd == 2) inv_2x2(d, sm.inv[tid]);
   }
   __syncthreads();
-  const int np = xi[kINp];
-  double* F = s.dpool + B->doff;
-  const double* Wg = s.dpool + B->woff;
   // L of the accepted pivots on the rows below the block
-  const int r = k + nbk + chunk * kThreads + tid;
   if (r < f) {
-    for (int p = 0; p < np;) {
-      if (sm.skind[p] == 1) {
-        F[r + (size_t)f * (k + p)] = Wg[(size_t)p * f + r] * sm.sinv[p];
-        p += 1;
-      } else {
-        double l0, l1;
-        l_2x2(sm.sd + 3 * p, Wg[(size_t)p * f + r], Wg[(size_t)(p + 1) * f + r], l0, l1);
-        F[r + (size_t)f * (k + p)] = l0;
-        F[r + (size_t)f * (k + p + 1)] = l1;
-        p += 2;
+    double* Fr = F + r + (size_t)f * k;
+#pragma unroll
+    for (int p = 0; p < kBlk; p++) {
+      if (p < np) {
+        const int kd = sm.skind[p];
+        double l = 0.0;
+        if (kd == 1) l = w[p] * sm.sinv[p];
+        if (p + 1 < kBlk && kd == 2) l = l_first(sm.inv[p], w[p], w[p + 1]);
+        if (p > 0 && kd == 3) l = l_second(sm.inv[p - 1], w[p - 1], w[p]);
+        Fr[(size_t)f * p] = l;
       }
     }
   }
@@ -860,61 +1086,66 @@ __device__ void phase_a_item(const DevState& s, const FactorParams& prm, BigFron
         v = sm.Ls[i][p];
       F[(k + i) + (size_t)f * (k + p)] = v;
     }
-    if (tid == 0) {
+    if (tid < 32) {
       // commit the panel (the other items of this front read only the
-      // scratch, never the descriptor)
+      // scratch, never the descriptor), a lane per pivot
       int* fv = s.ivars + B->ioff;
+      const int p = tid;
+      const int kd = p < np ? sm.skind[p] : 0;
       int npos = 0, nneg = 0;
-      double flops = 0.0;
-      for (int p = 0; p < np;) {
-        if (sm.skind[p] == 1) {
-          if (sm.sd[3 * p] >= 0.0)
-            npos++;
+      double fl = 0.0;
+      if (kd == 1) {
+        if (sm.sd[3 * p] >= 0.0)
+          npos = 1;
+        else
+          nneg = 1;
+        fl = 2.0 * (double)(f - k - p) * (p + 1);
+      } else if (kd == 2) {
+        const double d11 = sm.sd[3 * p], d21 = sm.sd[3 * p + 1], d22 = sm.sd[3 * p + 2];
+        const double det = d11 * d22 - d21 * d21;
+        if (det >= 0.0) {
+          if (d11 >= 0.0)
+            npos = 2;
           else
-            nneg++;
-          flops += 2.0 * (double)(f - k - p) * (p + 1);
-          p += 1;
+            nneg = 2;
         } else {
-          const double d11 = sm.sd[3 * p], d21 = sm.sd[3 * p + 1], d22 = sm.sd[3 * p + 2];
-          const double det = d11 * d22 - d21 * d21;
-          if (det >= 0.0) {
-            if (d11 >= 0.0)
-              npos += 2;
-            else
-              nneg += 2;
-          } else {
-            npos++;
-            nneg++;
-          }
-          fv[k + p] = -(fv[k + p] + 1);
-          fv[k + p + 1] = -(fv[k + p + 1] + 1);
-          flops += 4.0 * (double)(f - k - p) * (p + 2);
-          p += 2;
+          npos = 1;
+          nneg = 1;
         }
+        fl = 4.0 * (double)(f - k - p) * (p + 2);
       }
+      if (kd >= 2) fv[k + p] = -(fv[k + p] + 1);
       // candidates to delay: those that failed in the block while only
       // pivots that are now accepted preceded them, and the first pivot the
       // a-posteriori tests reject (positions decreasing); candidates that
       // failed after a rejected pivot are tried again
       const int acc = xi[kIAcc];
       const int ncand = xi[kINcand];
-      int nd = 0;
-      for (int q = nbk - 1; q >= acc; q--)
-        if (xi[kIDlt + q] >= 0 && xi[kIDlt + q] <= np) xi[kIDpos + nd++] = k + q;
-      if (np < acc) xi[kIDpos + nd++] = k + np;
-      xi[kIDcnt] = nd;
-      B->kstart = k;
-      B->kw = np;
-      B->k = k + np;
-      B->pending = nd;
-      B->npos += npos;
-      B->nneg += nneg;
-      B->flops += flops;
-      atomicAdd(s.flops + 1, flops);
-      atomicAdd(s.flops + 5, 1.0);
-      if (np < acc) atomicAdd(s.flops + 6, 1.0);
-      atomicAdd(s.flops + 7, (double)(nd - (np < acc ? 1 : 0)));
-      B->state = (nd == 0 && k + np >= ncand) ? 1 : 0;
+      const int dlt = (p >= acc && p < nbk) ? xi[kIDlt + p] : -1;
+      const unsigned late = __ballot_sync(0xffffffffu, dlt >= 0 && dlt <= np);
+      if ((late >> p) & 1u) xi[kIDpos + __popc(late >> p) - 1] = k + p;
+      const int nlate = __popc(late);
+      if (p == 0 && np < acc) xi[kIDpos + nlate] = k + np;
+      const int nd = nlate + (np < acc ? 1 : 0);
+      npos = __reduce_add_sync(0xffffffffu, npos);
+      nneg = __reduce_add_sync(0xffffffffu, nneg);
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) fl += __shfl_xor_sync(0xffffffffu, fl, d);
+      if (p == 0) {
+        xi[kIDcnt] = nd;
+        B->kstart = k;
+        B->kw = np;
+        B->k = k + np;
+        B->pending = nd;
+        B->npos += npos;
+        B->nneg += nneg;
+        B->flops += fl;
+        atomicAdd(s.flops + 1, fl);
+        atomicAdd(s.flops + 5, 1.0);
+        if (np < acc) atomicAdd(s.flops + 6, 1.0);
+        atomicAdd(s.flops + 7, (double)nlate);
+        B->state = (nd == 0 && k + np >= ncand) ? 1 : 0;
+      }
     }
   }
   __syncthreads();
@@ -922,128 +1153,187 @@ __device__ void phase_a_item(const DevState& s, const FactorParams& prm, BigFron
 
 // ---------------------------------------------------------------- phase U
 
-// One 64 x 64 lower tile of front B's trailing matrix at rows i0, columns
-// j0: the rank-kw update with the panel's L (columns ks..ks+kw) and W (Wg),
-// in FP64; k = ks + kw is the trailing matrix's first position. L is read
-// from the front's columns once committed, or (from_w) formed from W and
-// the panel's D as the commit forms it.
-__device__ void phase_u_tile(const DevState& s, const BigFront& B, int i0, int j0, int k, int kw,
-                             int ks, bool from_w, UpdSm& sm) {
+// One 64 x 64 lower tile of a front's trailing matrix at rows i0, columns j0:
+// the rank-kw update with the panel's L (columns ks..ks+kw) and W, in FP64;
+// k = ks + kw is the trailing matrix's first position. L is read from the
+// front's columns once committed, or (from_w) formed from W and the panel's D
+// as the commit forms it.
+//
+// The products run as mma.m8n8k4.f64, which adds its four products to the
+// accumulator one after another in the order of k, each with one rounding:
+// the sums are those of a loop of fused multiply-adds, at an eighth of the
+// instructions (the FP64 rate is the same, but a tile was bound by issuing
+// multiply-adds, operand loads and addresses). The next tile's loads are in
+// flight while one is computed.
+struct Tile {
+  double *F, *W, *X;
+  int f, i0, j0, k, kw, ks;
+};
+
+struct TileRegs {
+  static constexpr int kPer = kBigPanelMax * kTileU / kThreads;
+  double cur[4][2][2];  // this thread's entries: blocks of 8 rows, of 8 columns
+  // W (or L) at row i0 + tid % 64 of the columns 8 (tid / 64) - 1 .. + 8, and
+  // W at row j0 + tid % 64 of the columns 8 (tid / 64) ..
+  double pa[kPer + 2], pb[kPer];
+  double d0, d1, d2;  // of thread c < 32: pivot column c's D
+  int kd;
+};
+
+// warp w owns the tile's rows 32 (w % 2).. and columns 16 (w / 2)..; in a
+// block of 8 x 8 lane l holds row l / 4 and columns 2 (l % 4), + 1
+struct TileThread {
+  int row, col;
+  __device__ __forceinline__ TileThread() {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    row = 32 * (warp & 1) + (lane >> 2);
+    col = 16 * (warp >> 1) + 2 * (lane & 3);
+  }
+};
+
+__device__ __forceinline__ void load_tile(const Tile& t, bool from_w, TileRegs& g) {
   const int tid = threadIdx.x;
-  const int tx = tid & 15;
-  const int ty = tid >> 4;
-  const int f = B.f;
-  double* F = s.dpool + B.doff;
-  const double* W = s.dpool + B.woff;
-  if (from_w && tid < kBlk) {
-    const double* X = s.dpool + B.xoff;
-    const int kd = reinterpret_cast<const int*>(X + kXInt)[kIKind + tid];
-    sm.ukind[tid] = kd;
-    sm.ud[3 * tid] = X[kXD + 3 * tid];
-    sm.ud[3 * tid + 1] = X[kXD + 3 * tid + 1];
-    sm.ud[3 * tid + 2] = X[kXD + 3 * tid + 2];
-    sm.usinv[tid] = (kd == 1) ? 1.0 / X[kXD + 3 * tid] : 0.0;
-  }
-  double cur[4][4];
-#pragma unroll
-  for (int b = 0; b < 4; b++) {
-    const int j = j0 + ty + 16 * b;
-#pragma unroll
-    for (int a = 0; a < 4; a++) {
-      const int i = i0 + tx + 16 * a;
-      cur[a][b] = (j < f && i < f && i >= j) ? F[i + (size_t)f * j] : 0.0;
-    }
-  }
+  const int f = t.f;
   {
-    constexpr int kPer = kBigPanelMax * kTileU / kThreads;
-    double pa[kPer], pb[kPer];
+    const int rr = tid % kTileU, c0 = (tid / kTileU) * TileRegs::kPer;
+    const int i = t.i0 + rr, j = t.j0 + rr;
+    const double* pw = from_w ? t.W + i : t.F + i + (size_t)f * t.ks;
 #pragma unroll
-    for (int q = 0; q < kPer; q++) {
-      const int e = tid + kThreads * q;
-      const int c = e / kTileU;
-      const int rr = e - c * kTileU;
-      pa[q] = 0.0;
-      pb[q] = 0.0;
-      if (c < kw) {
-        if (i0 + rr < f)
-          pa[q] = from_w ? W[(size_t)c * f + i0 + rr] : F[i0 + rr + (size_t)f * (ks + c)];
-        if (j0 + rr < f) pb[q] = W[(size_t)c * f + j0 + rr];
-      }
+    for (int q = 0; q < TileRegs::kPer + 2; q++) {
+      const int c = c0 + q - 1;
+      const bool edge = q == 0 || q == TileRegs::kPer + 1;
+      g.pa[q] = (i < f && c >= 0 && c < t.kw && (!edge || from_w)) ? pw[(size_t)f * c] : 0.0;
     }
 #pragma unroll
-    for (int q = 0; q < kPer; q++) {
-      const int e = tid + kThreads * q;
-      const int c = e / kTileU;
-      const int rr = e - c * kTileU;
-      if (c < kw) {
-        sm.As[c][rr] = pa[q];
-        sm.Bs[c][rr] = pb[q];
-      }
-    }
+    for (int q = 0; q < TileRegs::kPer; q++)
+      g.pb[q] = (j < f && c0 + q < t.kw) ? t.W[j + (size_t)f * (c0 + q)] : 0.0;
   }
-  __syncthreads();
-  if (from_w) {
-    // L = W D^-1 on the tile's rows, the commit's expressions
-    for (int e = tid; e < kw * kTileU; e += kThreads) {
-      const int c = e / kTileU, rr = e - c * kTileU;
-      const int kd = sm.ukind[c];
-      if (kd == 1) {
-        sm.As[c][rr] = sm.As[c][rr] * sm.usinv[c];
-      } else if (kd == 2) {
-        double l0, l1;
-        l_2x2(sm.ud + 3 * c, sm.As[c][rr], sm.As[c + 1][rr], l0, l1);
-        sm.As[c][rr] = l0;
-        sm.As[c + 1][rr] = l1;
+  g.kd = 0;
+  g.d0 = g.d1 = g.d2 = 0.0;
+  if (from_w && tid < kBlk) {
+    g.kd = xint(t.X)[kIKind + tid];
+    g.d0 = t.X[kXD + 3 * tid];
+    g.d1 = t.X[kXD + 3 * tid + 1];
+    g.d2 = t.X[kXD + 3 * tid + 2];
+  }
+  const TileThread me;
+#pragma unroll
+  for (int b = 0; b < 2; b++)
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const int j = t.j0 + me.col + 8 * b + e;
+      const double* col = t.F + (size_t)f * j;
+#pragma unroll
+      for (int a = 0; a < 4; a++) {
+        const int i = t.i0 + me.row + 8 * a;
+        g.cur[a][b][e] = (j < f && i < f && i >= j) ? col[i] : 0.0;
       }
+    }
+}
+
+// the panel parts of g into shared memory, L formed (all threads; ends with a
+// barrier). same: the tile is of the same front as the one before, whose D^-1
+// is in place.
+__device__ __forceinline__ void stage_tile(const Tile& t, bool from_w, bool same,
+                                           const TileRegs& g, UpdSm& sm) {
+  const int tid = threadIdx.x;
+  if (from_w && !same) {
+    if (tid < kBlk) {
+      const double d[3] = {g.d0, g.d1, g.d2};
+      sm.ukind[tid] = g.kd;
+      sm.usinv[tid] = (g.kd == 1) ? 1.0 / g.d0 : 0.0;
+      if (g.kd == 2) inv_2x2(d, sm.ud + 3 * tid);
     }
     __syncthreads();
   }
-  double acc[4][4];
+  const int rr = tid % kTileU, c0 = (tid / kTileU) * TileRegs::kPer;
+#pragma unroll
+  for (int q = 0; q < TileRegs::kPer; q++) {
+    const int c = c0 + q;
+    double l = g.pa[q + 1];
+    if (from_w) {
+      // L = W D^-1 on the tile's rows, the commit's expressions
+      const int kd = c < t.kw ? sm.ukind[c] : 0;
+      if (kd == 1)
+        l = g.pa[q + 1] * sm.usinv[c];
+      else if (kd == 2)
+        l = l_first(sm.ud + 3 * c, g.pa[q + 1], g.pa[q + 2]);
+      else if (kd == 3)
+        l = l_second(sm.ud + 3 * (c - 1), g.pa[q], g.pa[q + 1]);
+    }
+    sm.As[c][rr] = l;
+    sm.Bs[c][rr] = g.pb[q];
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ void finish_tile(const Tile& t, const double (&cur)[4][2][2],
+                                            const UpdSm& sm) {
+  const int lane = threadIdx.x & 31;
+  const int f = t.f, k = t.k;
+  const TileThread me;
+  const int row0 = me.row, c16 = me.col - 2 * (lane & 3) + (lane >> 2);
+  double acc[4][2][2];
 #pragma unroll
   for (int a = 0; a < 4; a++)
 #pragma unroll
-    for (int b = 0; b < 4; b++) acc[a][b] = 0.0;
-  for (int c = 0; c < kw; c++) {
-    double av[4], bv[4];
+    for (int b = 0; b < 2; b++) acc[a][b][0] = acc[a][b][1] = 0.0;
+  const double* ap = &sm.As[lane & 3][row0];
+  const double* bp = &sm.Bs[lane & 3][c16];
+  // columns at and beyond kw are zeros
+  for (int c = 0; c < t.kw; c += 4) {
+    double av[4], bv[2];
 #pragma unroll
-    for (int a = 0; a < 4; a++) av[a] = sm.As[c][tx + 16 * a];
+    for (int a = 0; a < 4; a++) av[a] = ap[c * kTileLdU + 8 * a];
 #pragma unroll
-    for (int b = 0; b < 4; b++) bv[b] = sm.Bs[c][ty + 16 * b];
+    for (int b = 0; b < 2; b++) bv[b] = bp[c * kTileLdU + 8 * b];
 #pragma unroll
     for (int a = 0; a < 4; a++)
 #pragma unroll
-      for (int b = 0; b < 4; b++) acc[a][b] = fma(av[a], bv[b], acc[a][b]);
+      for (int b = 0; b < 2; b++)
+        asm volatile(
+            "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+            : "+d"(acc[a][b][0]), "+d"(acc[a][b][1])
+            : "d"(av[a]), "d"(bv[b]));
   }
 #pragma unroll
-  for (int b = 0; b < 4; b++) {
-    const int j = j0 + ty + 16 * b;
-    if (j >= f) continue;
+  for (int b = 0; b < 2; b++)
 #pragma unroll
-    for (int a = 0; a < 4; a++) {
-      const int i = i0 + tx + 16 * a;
-      if (i < f && i >= j) F[i + (size_t)f * j] = cur[a][b] - acc[a][b];
-    }
-  }
-  if (j0 == k) {
-    // the next panel's columns [k, k + 32): their largest magnitude over the
-    // rows below the next block, for its first test (the 16 threads with
-    // the same ty are one half-warp)
-    unsigned long long* nxt =
-        reinterpret_cast<unsigned long long*>(s.dpool + B.xoff + kAppNextColmax);
-#pragma unroll
-    for (int b = 0; b < 2; b++) {
-      double m = 0.0;
+    for (int e = 0; e < 2; e++) {
+      const int j = t.j0 + me.col + 8 * b + e;
+      double* col = t.F + (size_t)f * j;
 #pragma unroll
       for (int a = 0; a < 4; a++) {
-        const int i = i0 + tx + 16 * a;
-        if (i < f && i >= k + kBigPanelMax) m = fmax(m, fabs(cur[a][b] - acc[a][b]));
+        const int i = t.i0 + me.row + 8 * a;
+        if (j < f && i < f && i >= j) col[i] = cur[a][b][e] - acc[a][b][e];
       }
-#pragma unroll
-      for (int o = 1; o < 16; o <<= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-      const int j = j0 + ty + 16 * b;
-      if (tx == 0 && j < f && m > 0.0)
-        atomicMax(nxt + (ty + 16 * b), (unsigned long long)__double_as_longlong(m));
     }
+  if (t.j0 == k && me.col < kBigPanelMax) {
+    // the next panel's columns [k, k + 32): their largest magnitude over the
+    // rows below the next block, for its first test (as bits; NaN entries do
+    // not take part)
+    unsigned long long* nxt =
+        reinterpret_cast<unsigned long long*>(t.X + kAppNextColmax);
+#pragma unroll
+    for (int b = 0; b < 2; b++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        unsigned long long m = 0;
+#pragma unroll
+        for (int a = 0; a < 4; a++) {
+          const int i = t.i0 + me.row + 8 * a;
+          const unsigned long long x =
+              (unsigned long long)__double_as_longlong(fabs(cur[a][b][e] - acc[a][b][e]));
+          if (i < f && i >= k + kBigPanelMax && x <= kInfBits && x > m) m = x;
+        }
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) {
+          const unsigned long long x = __shfl_xor_sync(0xffffffffu, m, o);
+          if (x > m) m = x;
+        }
+        const int jj = me.col + 8 * b + e;
+        if ((lane >> 2) == 0 && k + jj < f && m > 0) atomicMax(nxt + jj, m);
+      }
   }
   __syncthreads();
 }
@@ -1057,11 +1347,16 @@ __device__ __forceinline__ long long tri_tiles(const BigFront& B, int tile) {
   return tri_tiles_rows(B.f - B.k, tile);
 }
 
-__device__ __forceinline__ void tri_decode(long long lt, int& I, int& J) {
-  I = (int)((sqrt(8.0 * (double)lt + 1.0) - 1.0) * 0.5);
-  while ((long long)(I + 1) * (I + 2) / 2 <= lt) I++;
-  while ((long long)I * (I + 1) / 2 > lt) I--;
-  J = (int)(lt - (long long)I * (I + 1) / 2);
+// tile lt of a lower triangle of T x T tiles, column by column: the CTAs that
+// run at the same time then cover long stretches of the same columns (DRAM
+// pages), and the tiles of the next panel's columns come first
+__device__ __forceinline__ void tri_decode(long long lt, int T, int& I, int& J) {
+  const int r = (int)((long long)T * (T + 1) / 2 - 1 - lt);  // row by row from the end
+  int a = (int)((sqrtf(8.0f * (float)r + 1.0f) - 1.0f) * 0.5f);
+  while ((long long)(a + 1) * (a + 2) / 2 <= r) a++;
+  while ((long long)a * (a + 1) / 2 > r) a--;
+  J = T - 1 - a;
+  I = T - 1 - (int)(r - (long long)a * (a + 1) / 2);
 }
 
 // Mixed precision: a 128 x 128 tile (I, J) of the trailing matrix. Tiles of
@@ -1086,8 +1381,14 @@ __device__ int phase_u_tile_mixed(const DevState& s, const BigFront& B, int I, i
   for (int a = 0; a < 2; a++)
     for (int b = 0; b < 2; b++) {
       const int si = i0 + a * kTileU, sj = j0 + b * kTileU;
-      if (si < f && sj < f && si + kTileU - 1 >= sj)
-        phase_u_tile(s, B, si, sj, B.k, B.kw, B.kstart, false, sm);
+      if (si < f && sj < f && si + kTileU - 1 >= sj) {
+        const Tile t = {s.dpool + B.doff, s.dpool + B.woff, s.dpool + B.xoff, f, si, sj,
+                        B.k,             B.kw,             B.kstart};
+        TileRegs g;
+        load_tile(t, false, g);
+        stage_tile(t, false, false, g, sm);
+        finish_tile(t, g.cur, sm);
+      }
     }
   return 0;
 }
@@ -1099,7 +1400,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                      int max_steps, int* done, int* meta) {
   int* counters = meta + 21;
   cg::grid_group grid = cg::this_grid();
-  extern __shared__ __align__(1024) unsigned char dsm[];
+  extern __shared__ __align__(1024) unsigned char dsm0[];
+  Info* info = reinterpret_cast<Info*>(dsm0);
+  unsigned char* dsm = dsm0 + kInfoBytes;
   __shared__ Prefix P;
   __shared__ __align__(8) uint64_t mbar;
   __shared__ uint32_t tmem_slot;
@@ -1118,17 +1421,21 @@ __global__ void __launch_bounds__(kThreads, 1)
     asm volatile("tcgen05.fence::after_thread_sync;" ::);
     tmem = tmem_slot;
   }
+  // where the fronts are (more of them than fit are looked up in every step)
+  if (nl <= kChunkFronts)
+    for (int i = tid; i < nl; i += kThreads) front_place(s, s.big[list[i]], info[i]);
   int step = 1;
   for (; step <= max_steps; step++) {
     // ---- D: one warp per front
     {
       WarpDiag& w = reinterpret_cast<WarpDiag*>(dsm)[warp];
+      WarpDiag& w0 = reinterpret_cast<WarpDiag*>(dsm)[0];
       if (blockIdx.x == 0 && tid == 0) counters[(step + 1) & 1] = 0;
       if (nl <= (int)gridDim.x) {
         // a CTA per front: its threads apply the delays, warp 0 the block
         if ((int)blockIdx.x < nl) {
           BigFront* B = s.big + list[blockIdx.x];
-          if (phase_d_prepare<kThreads>(s, B, done, meta, tid) && warp == 0) {
+          if (phase_d_prepare<kThreads>(s, B, done, meta, tid, w0) && warp == 0) {
             phase_d_block(s, prm, B, step, w);
             if (tid == 0) atomicAdd(counters + (step & 1), 1);
           }
@@ -1136,7 +1443,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       } else {
         for (int i = gwarp; i < nl; i += nwarp) {
           BigFront* B = s.big + list[i];
-          if (phase_d_prepare<32>(s, B, done, meta, tid & 31)) {
+          if (phase_d_prepare<32>(s, B, done, meta, tid & 31, w)) {
             phase_d_block(s, prm, B, step, w);
             if ((tid & 31) == 0) atomicAdd(counters + (step & 1), 1);
           }
@@ -1148,14 +1455,14 @@ __global__ void __launch_bounds__(kThreads, 1)
     // ---- R: row chunks of the active fronts
     for (int c0 = 0; c0 < nl; c0 += kChunkFronts) {
       const int n = min(kChunkFronts, nl - c0);
-      const long long total = front_prefix(
-          P, n, [&](int i) { return (long long)row_chunks(s, s.big[list[c0 + i]], step); });
+      const long long total = front_prefix(P, n, [&](int i) {
+        if (nl > kChunkFronts) front_place(s, s.big[list[c0 + i]], info[i]);
+        return (long long)front_step(step, info[i]);
+      });
       RowsSm& sm = *reinterpret_cast<RowsSm*>(dsm);
       for (long long t = blockIdx.x; t < total; t += gridDim.x) {
         const int fi = item_front(P, n, t);
-        const BigFront& B = s.big[list[c0 + fi]];
-        const int nchunk = (int)(P.ptr[fi + 1] - P.ptr[fi]);
-        phase_r_item(s, prm, B, (int)(t - P.ptr[fi]), nchunk, sm);
+        phase_r_item(prm, info[fi], (int)(t - P.ptr[fi]), sm);
       }
       __syncthreads();
     }
@@ -1168,28 +1475,58 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int c0 = 0; c0 < nl; c0 += kChunkFronts) {
         const int n = min(kChunkFronts, nl - c0);
         const long long total = front_prefix(P, n, [&](int i) {
-          const BigFront& B = s.big[list[c0 + i]];
-          const int ra = row_chunks(s, B, step);
-          if (ra == 0) return 0ll;
-          const int* xi = xint(s.dpool + B.xoff);
-          const int np = xi[kINp];
-          return (long long)ra + (np > 0 ? tri_tiles_rows(B.f - (xi[kIK] + np), kTileU) : 0ll);
-        });
-        for (long long t = blockIdx.x; t < total; t += gridDim.x) {
-          const int fi = item_front(P, n, t);
-          BigFront* B = s.big + list[c0 + fi];
-          const long long it = t - P.ptr[fi];
-          const int ra = row_chunks(s, *B, step);
-          if (it < ra) {
-            phase_a_item(s, prm, B, (int)it, *reinterpret_cast<RowsSm*>(dsm));
-          } else {
-            const int* xi = xint(s.dpool + B->xoff);
-            const int ks = xi[kIK], np = xi[kINp];
-            int I, J;
-            tri_decode(it - ra, I, J);
-            phase_u_tile(s, *B, ks + np + I * kTileU, ks + np + J * kTileU, ks + np, np, ks, true,
-                         *reinterpret_cast<UpdSm*>(dsm));
+          Info& o = info[i];
+          if (nl > kChunkFronts) {
+            front_place(s, s.big[list[c0 + i]], o);
+            front_step(step, o);
           }
+          if (o.rows == 0) return 0ll;
+          o.np = xint(o.X)[kINp];
+          return o.rows + (o.np > 0 ? tri_tiles_rows(o.f - (o.k + o.np), kTileU) : 0ll);
+        });
+        UpdSm& sm = *reinterpret_cast<UpdSm*>(dsm);
+        // the CTA's items in turn; a tile's loads are issued before the tile
+        // before it is computed
+        auto tile_of = [&](long long t, Tile& o) {  // false: a row chunk
+          const int fi = item_front(P, n, t);
+          const Info& q = info[fi];
+          const long long it = t - P.ptr[fi];
+          if (it < q.rows) return false;
+          int I, J;
+          const int k = q.k + q.np;
+          tri_decode(it - q.rows, (q.f - k + kTileU - 1) / kTileU, I, J);
+          o = {q.F, q.W, q.X, q.f, k + I * kTileU, k + J * kTileU, k, q.np, q.k};
+          return true;
+        };
+        Tile tile;
+        TileRegs regs;
+        bool have = false;
+        const double* last = nullptr;  // whose D^-1 is in shared memory
+        for (long long t = blockIdx.x; t < total; t += gridDim.x) {
+          if (!have) {
+            if (!tile_of(t, tile)) {
+              const int fi = item_front(P, n, t);
+              phase_a_item(s, s.big + list[c0 + fi], info[fi], (int)(t - P.ptr[fi]),
+                           *reinterpret_cast<RowsSm*>(dsm));
+              last = nullptr;
+              continue;
+            }
+            load_tile(tile, true, regs);
+          }
+          stage_tile(tile, true, tile.X == last, regs, sm);
+          last = tile.X;
+          const Tile now = tile;
+          double cur[4][2][2];
+#pragma unroll
+          for (int a = 0; a < 4; a++)
+#pragma unroll
+            for (int b = 0; b < 2; b++) {
+              cur[a][b][0] = regs.cur[a][b][0];
+              cur[a][b][1] = regs.cur[a][b][1];
+            }
+          have = t + gridDim.x < total && tile_of(t + gridDim.x, tile);
+          if (have) load_tile(tile, true, regs);
+          finish_tile(now, cur, sm);
         }
         __syncthreads();
       }
@@ -1199,12 +1536,19 @@ __global__ void __launch_bounds__(kThreads, 1)
     // ---- A: the same items; the first one of a front commits the panel
     for (int c0 = 0; c0 < nl; c0 += kChunkFronts) {
       const int n = min(kChunkFronts, nl - c0);
-      const long long total = front_prefix(
-          P, n, [&](int i) { return (long long)row_chunks(s, s.big[list[c0 + i]], step); });
+      const long long total = front_prefix(P, n, [&](int i) {
+        Info& o = info[i];
+        if (nl > kChunkFronts) {
+          front_place(s, s.big[list[c0 + i]], o);
+          front_step(step, o);
+        }
+        if (o.rows > 0) o.np = xint(o.X)[kINp];
+        return (long long)o.rows;
+      });
       RowsSm& sm = *reinterpret_cast<RowsSm*>(dsm);
       for (long long t = blockIdx.x; t < total; t += gridDim.x) {
         const int fi = item_front(P, n, t);
-        phase_a_item(s, prm, s.big + list[c0 + fi], (int)(t - P.ptr[fi]), sm);
+        phase_a_item(s, s.big + list[c0 + fi], info[fi], (int)(t - P.ptr[fi]), sm);
       }
       __syncthreads();
     }
@@ -1222,7 +1566,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int fi = item_front(P, n, t);
         const BigFront& B = s.big[list[c0 + fi]];
         int I, J;
-        tri_decode(t - P.ptr[fi], I, J);
+        tri_decode(t - P.ptr[fi], (B.f - B.k + umma::kTileM - 1) / umma::kTileM, I, J);
         if (!tc_fail) {
           // the tensor-core operands share the dynamic shared memory with
           // the FP64 tiles' panels (a tile uses one or the other)

@@ -1347,6 +1347,8 @@ __global__ void __launch_bounds__(kFactorThreads, kMax == 1 ? 4 : kMax == 2 ? 3 
 
 }  // namespace
 
+int factor_variant(int fmax) { return row_chunks(fmax); }
+
 size_t factor_smem_bytes(int f) {
   // the front (ld = f | 1), the travelling columns, the variables and their
   // positions at assembly

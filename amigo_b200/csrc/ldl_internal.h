@@ -259,6 +259,8 @@ void launch_factor_level(const DevPlan& p, const DevState& s, const int* nodes, 
                          const double* diag);
 cudaError_t configure_factor_kernels();
 size_t factor_smem_bytes(int f);
+// the kernel variant that a launch for fronts up to fmax takes
+int factor_variant(int fmax);
 
 // Big-front pipeline for one level (see big.cu).
 struct BigLevelInfo {
