@@ -96,7 +96,11 @@ struct b200ldl_assembly {
   int n = 0, nnz = 0;
   long long nvals = 0;    // block values expected (sum over groups of nelem * ncomp^2)
   long long dropped = 0;  // contributions outside the pattern
-  std::vector<long long> ptr, src;  // the plan, host copy
+  // the plan, host copy: 32-bit where it fits
+  std::vector<long long> ptr, src;
+  std::vector<int> ptr32, src32;
+  bool narrow = false;
+  long long kept() const { return narrow ? (long long)src32.size() : (long long)src.size(); }
   DevArr<long long> d_ptr, d_src;  // for factorizations from element blocks
   DevArr<int> d_ptr32, d_src32;    // for the gather, where the plan fits
   bool uploaded = false;
@@ -125,27 +129,18 @@ inline long long find_entry(const int* rowp, const int* cols, int row, int col) 
   return (it != e && *it == col) ? (long long)(it - cols) : -1;
 }
 
+template <typename T>
+cudaError_t to_device(DevArr<T>& d, const std::vector<T>& h) {
+  cudaError_t e = cudaMalloc(&d.ptr, std::max<size_t>(1, h.size()) * sizeof(T));
+  if (e == cudaSuccess && !h.empty())
+    e = cudaMemcpy(d.ptr, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice);
+  return e;
+}
+
 int upload(b200ldl_assembly* a) {
   if (a->uploaded) return 0;
-  const size_t np = a->ptr.size(), ns = std::max<size_t>(1, a->src.size());
-  cudaError_t e = cudaMalloc(&a->d_ptr.ptr, np * sizeof(long long));
-  if (e == cudaSuccess) e = cudaMalloc(&a->d_src.ptr, ns * sizeof(long long));
-  if (e == cudaSuccess)
-    e = cudaMemcpy(a->d_ptr.ptr, a->ptr.data(), np * sizeof(long long), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && !a->src.empty())
-    e = cudaMemcpy(a->d_src.ptr, a->src.data(), a->src.size() * sizeof(long long),
-                   cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && a->nvals <= 2147483647LL && a->src.size() <= 2147483647u) {
-    const std::vector<int> p32(a->ptr.begin(), a->ptr.end());
-    const std::vector<int> s32(a->src.begin(), a->src.end());
-    e = cudaMalloc(&a->d_ptr32.ptr, np * sizeof(int));
-    if (e == cudaSuccess) e = cudaMalloc(&a->d_src32.ptr, ns * sizeof(int));
-    if (e == cudaSuccess)
-      e = cudaMemcpy(a->d_ptr32.ptr, p32.data(), np * sizeof(int), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && !s32.empty())
-      e = cudaMemcpy(a->d_src32.ptr, s32.data(), s32.size() * sizeof(int),
-                     cudaMemcpyHostToDevice);
-  }
+  cudaError_t e = a->narrow ? to_device(a->d_ptr32, a->ptr32) : to_device(a->d_ptr, a->ptr);
+  if (e == cudaSuccess) e = a->narrow ? to_device(a->d_src32, a->src32) : to_device(a->d_src, a->src);
   if (e != cudaSuccess) return afail(a, -3, "CUDA error: %s", cudaGetErrorString(e));
   a->uploaded = true;
   return 0;
@@ -198,6 +193,8 @@ int b200ldl_assembly_create(b200ldl_assembly_t* out, int n, const int* rowp, con
             }
             if (pass == 0)
               cnt[p + 1]++;
+            else if (a->narrow)
+              a->src32[cnt[p]++] = (int)(off + ((long long)e * m + j) * m + i);
             else
               a->src[cnt[p]++] = off + ((long long)e * m + j) * m + i;
           }
@@ -208,7 +205,14 @@ int b200ldl_assembly_create(b200ldl_assembly_t* out, int n, const int* rowp, con
     if (pass == 0) {
       for (int p = 0; p < a->nnz; p++) cnt[p + 1] += cnt[p];
       a->ptr = cnt;
-      a->src.assign((size_t)cnt[a->nnz], 0);
+      a->narrow = a->nvals <= 2147483647LL && cnt[a->nnz] <= 2147483647LL;
+      if (a->narrow) {
+        a->ptr32.assign(a->ptr.begin(), a->ptr.end());
+        std::vector<long long>().swap(a->ptr);
+        a->src32.assign((size_t)cnt[a->nnz], 0);
+      } else {
+        a->src.assign((size_t)cnt[a->nnz], 0);
+      }
     }
   }
   return 0;
@@ -218,7 +222,7 @@ int b200ldl_assembly_values(b200ldl_assembly_t a, const double* blocks, double* 
                             void* stream) {
   if (!a) return -1;
   if (a->nnz > 0 && !vals) return afail(a, -1, "vals is null");
-  if (!a->src.empty() && !blocks) return afail(a, -1, "blocks is null");
+  if (a->kept() > 0 && !blocks) return afail(a, -1, "blocks is null");
   if (a->nnz == 0) return 0;
   const int st = upload(a);
   if (st != 0) return st;
@@ -226,7 +230,7 @@ int b200ldl_assembly_values(b200ldl_assembly_t a, const double* blocks, double* 
   const int per_cta = threads * kPer;
   const int grid = std::max(1, std::min((a->nnz - 1) / per_cta + 1, 148 * 64));
   const cudaStream_t st_ = static_cast<cudaStream_t>(stream);
-  if (a->d_ptr32.ptr)
+  if (a->narrow)
     csr_gather_kernel<<<grid, threads, 0, st_>>>(a->nnz, a->d_ptr32.ptr, a->d_src32.ptr, blocks,
                                                  vals);
   else
@@ -238,15 +242,20 @@ int b200ldl_assembly_values(b200ldl_assembly_t a, const double* blocks, double* 
 
 int b200ldl_assembly_info(b200ldl_assembly_t a, long long* out, int nout) {
   if (!a || !out) return -1;
-  const long long v[4] = {(long long)a->src.size(), a->dropped, a->nvals, (long long)a->nnz};
+  const long long v[4] = {a->kept(), a->dropped, a->nvals, (long long)a->nnz};
   for (int t = 0; t < nout && t < 4; t++) out[t] = v[t];
   return 0;
 }
 
 int b200ldl_assembly_plan(b200ldl_assembly_t a, long long* ptr, long long* src) {
   if (!a) return -1;
-  if (ptr) std::copy(a->ptr.begin(), a->ptr.end(), ptr);
-  if (src) std::copy(a->src.begin(), a->src.end(), src);
+  if (a->narrow) {
+    if (ptr) std::copy(a->ptr32.begin(), a->ptr32.end(), ptr);
+    if (src) std::copy(a->src32.begin(), a->src32.end(), src);
+  } else {
+    if (ptr) std::copy(a->ptr.begin(), a->ptr.end(), ptr);
+    if (src) std::copy(a->src.begin(), a->src.end(), src);
+  }
   return 0;
 }
 
@@ -260,9 +269,15 @@ void b200ldl_assembly_destroy(b200ldl_assembly_t a) { delete a; }
 
 namespace b200ldl {
 
-int assembly_device_plan(const ::b200ldl_assembly* a, int* n, int* nnz, const long long** ptr,
+int assembly_device_plan(::b200ldl_assembly* a, int* n, int* nnz, const long long** ptr,
                          const long long** src) {
-  if (!a || !a->d_ptr.ptr) return -1;
+  if (!a || !a->uploaded) return -1;
+  if (!a->d_ptr.ptr) {
+    // the fronts' scattered reads take 64-bit indices
+    const std::vector<long long> p(a->ptr32.begin(), a->ptr32.end());
+    const std::vector<long long> q(a->src32.begin(), a->src32.end());
+    if (to_device(a->d_src, q) != cudaSuccess || to_device(a->d_ptr, p) != cudaSuccess) return -1;
+  }
   *n = a->n;
   *nnz = a->nnz;
   *ptr = a->d_ptr.ptr;

@@ -366,7 +366,7 @@ void launch_perturb_diag(int n, const double* diag, const unsigned char* cls, do
 
 // The device copy of an assembly plan (assembly.cu): its pattern's size and
 // the per-CSR-entry contribution lists. Returns 0, or -1 without a plan.
-int assembly_device_plan(const ::b200ldl_assembly* a, int* n, int* nnz, const long long** ptr,
+int assembly_device_plan(::b200ldl_assembly* a, int* n, int* nnz, const long long** ptr,
                          const long long** src);
 
 }  // namespace b200ldl
