@@ -773,7 +773,7 @@ void level_fronts(b200ldl_t h) {
       const int node = h->hp_level_nodes[q];
       const int fn = f[node];
       h->level_fmax[l] = std::max(h->level_fmax[l], fn);
-      if (fn >= kSolveBigFront && solve_big_fits(fn)) {
+      if (fn >= kSolveBigFront && solve_big_rhs(fn) > 0) {
         big.push_back(node);
         run.big_fmax = std::max(run.big_fmax, fn);
         continue;
@@ -808,7 +808,9 @@ void level_fronts(b200ldl_t h) {
 // launches are asynchronous; finish_solve waits for them.
 void run_solve(b200ldl_t h, int nrhs, double* x, int ldx) {
   if (h->fmax == 0) level_fronts(h);
-  const int chunk = solve_rhs_chunk(h->fmax, nrhs);
+  int chunk = solve_rhs_chunk(h->fmax, nrhs);
+  for (const auto& r : h->solve_runs)
+    if (r.big_count > 0) chunk = std::min(chunk, solve_big_rhs(r.big_fmax));
   if (chunk < 1) throw std::runtime_error("front too large for the solve kernels");
   const size_t need = (size_t)h->used[2] * nrhs;
   if (h->d_upool.count < need) CK(h->d_upool.alloc(need));

@@ -333,7 +333,8 @@ cudaError_t configure_solve_kernels();
 // Supernodes with fronts of at least kSolveBigFront rows are solved by a
 // 16-CTA cluster each (solve_big.cu) when their vectors fit its shared memory.
 constexpr int kSolveBigFront = 1024;
-bool solve_big_fits(int f);
+// Right-hand sides per launch for fronts of f rows, 0 if not even one fits.
+int solve_big_rhs(int f);
 cudaError_t configure_solve_big_kernels();
 cudaError_t launch_forward_big(const DevPlan& p, const DevState& s, const SolveSpan& sp, double* x,
                                int ldx, int nrhs, int r0, int nr, double* upool,

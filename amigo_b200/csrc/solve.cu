@@ -33,6 +33,7 @@
 // eight right-hand sides: 11.9 ms with a launch per level and sweep, 3.1 ms
 // now; one right-hand side of 512 such systems: 9.8 and 2.8 ms.
 #include "ldl_internal.h"
+#include "solve_common.cuh"
 
 namespace b200ldl {
 
@@ -262,7 +263,7 @@ __device__ __forceinline__ void stage_factor(double* Ls, int ld, const double* L
 template <int kNr>
 __device__ __forceinline__ bool forward_node(const DevPlan& p, const DevState& s,
                                              const SolveArgs& a, int node, double* sm,
-                                             int* sh_fail) {
+                                             int* sh_fail, ChildBatch* kids) {
   constexpr int kLd = kVld<kNr>;
   const int tid = threadIdx.x;
   const int lane = tid & 31;
@@ -281,17 +282,16 @@ __device__ __forceinline__ bool forward_node(const DevPlan& p, const DevState& s
   const int kb = p.kid_ptr[node];
   const int ke = p.kid_ptr[node + 1];
   const long long uoff = s.u_off[node];
-  // the first child's place in the update vectors, before the wait
-  int ch = 0, nd = 0, mc = 0, cptr = 0;
+  // an only child's place in the update vectors, before the wait
+  int nd = 0, mc = 0, cptr = 0;
   long long cu = 0;
-  auto child = [&](int c) {
-    ch = p.kids[c];
+  if (ke - kb == 1) {
+    const int ch = p.kids[kb];
     nd = s.ndel[ch];
     mc = s.f[ch] - s.npiv[ch];
     cu = s.u_off[ch];
     cptr = p.cptr[ch];
-  };
-  if (kb < ke) child(kb);
+  }
   double* tile = sm;                                    // [2][kBlk][kTileLd], or the factor
   double* v = tile + a.stage_cap;                       // [f][kLd], post-pivot order
   int* post_of = reinterpret_cast<int*>(v + (size_t)kLd * f);  // [f]
@@ -331,9 +331,11 @@ __device__ __forceinline__ bool forward_node(const DevPlan& p, const DevState& s
   }
   __syncthreads();
   if (*sh_fail) return false;
+  if (ke - kb > 1)
+    add_children<kNr>(p, s, *kids, kb, ke, ns, nd_in, a.upool, a.nrhs, a.r0, nr, post_of,
+                      [&](int q, int r, double u) { v[q * kLd + r] += u; });
   int off = ns;
-  for (int c = kb; c < ke; c++) {
-    if (c > kb) child(c);
+  for (int c = kb; c < ke && ke - kb == 1; c++) {
     const double* uc = a.upool + cu * a.nrhs + (size_t)a.r0 * mc;
     const int* cm = p.cmap + cptr;
     for (int t = tid; t < mc; t += kSolveThreads) {
@@ -596,6 +598,7 @@ __global__ void __launch_bounds__(kSolveThreads, 2)
     solve_kernel(DevPlan p, DevState s, SolveArgs a) {
   extern __shared__ __align__(16) double sm[];
   __shared__ int sh_item, sh_fail;
+  __shared__ ChildBatch kids;
   const int items = a.sweeps == 3 ? 2 * a.count : a.count;
   if (threadIdx.x == 0) sh_fail = 0;
   for (;;) {
@@ -605,7 +608,7 @@ __global__ void __launch_bounds__(kSolveThreads, 2)
     if (item >= items) return;
     bool ok;
     if ((a.sweeps & 1) && item < a.count)
-      ok = forward_node<kNr>(p, s, a, a.nodes[item], sm, &sh_fail);
+      ok = forward_node<kNr>(p, s, a, a.nodes[item], sm, &sh_fail, &kids);
     else
       ok = backward_node<kNr>(p, s, a, a.nodes[items - 1 - item], sm, &sh_fail);
     if (!ok) {
