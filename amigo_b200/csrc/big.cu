@@ -154,57 +154,116 @@ __global__ void __launch_bounds__(256) big_assemble_kernel(DevPlan p, DevState s
       F[r + (size_t)f * p.scat_col[e]] += csr_value(s, vals, p.scat_csr[e]);
     }
   }
-  // the children's contribution blocks, one child after another
+  // The children's contribution blocks, one child after another. A child is
+  // mostly small (tens of rows) and there are up to 256 of them, so what it
+  // costs is latency: the children's sizes and places are looked up 32 at a
+  // time, and what a warp adds first for a child (positions and values of up
+  // to 128 rows of its first column) is loaded while the child before is
+  // added, which leaves a barrier and one read-modify-write of the front per
+  // child (hex elasticity 11^3 with a dense row: 10.5 -> 8.9 ms a
+  // factorization; plane stress 256 x 256: 32.6 -> 31.0).
+  __shared__ struct {
+    const double* cb[32];
+    const int* cm[32];
+    int m[32], nd[32], cld[32], off[32];
+    int next_off;
+  } kid;
   const int kb = p.kid_ptr[node];
   const int ke = p.kid_ptr[node + 1];
-  int off = ns;  // first position of this child's delayed rows
-  for (int q = kb; q < ke; q++) {
-    asm_sync<CL>();
-    const int ch = p.kids[q];
-    const int nd = s.ndel[ch];
-    const int m = s.f[ch] - s.npiv[ch];
-    const double* cb = s.dpool + s.cb_off[ch];
-    const int cld = s.cb_ld[ch];
-    const int* cm = p.cmap + p.cptr[ch];
-    for (int r2 = rank * kW + warp; r2 < m; r2 += CL * kW) {
-      int p2;
-      if (r2 < nd) {
-        p2 = off + r2;
-      } else {
-        p2 = cm[r2 - nd];
-        if (p2 >= ns) p2 += nd_in;
-      }
-      const double* col = cb + (size_t)cld * r2;
-      // four entries per lane pass: their loads (map, value, front) are in
-      // flight together before the read-modify-writes
-      for (int rb = r2 + lane; rb < m; rb += 128) {
-        double* dst[4];
-        double val[4];
+  if (threadIdx.x == 0) kid.next_off = ns;  // first position of the delayed rows
+  auto place = [&](int c, int r) {
+    const int nd = kid.nd[c];
+    int q;
+    if (r < nd) {
+      q = kid.off[c] + r;
+    } else {
+      q = kid.cm[c][r - nd];
+      if (q >= ns) q += nd_in;
+    }
+    return q;
+  };
+  struct Adds {
+    double* dst[4];
+    double val[4];
+  };
+  // rows rb, rb + 32, .. of column r2 of child c
+  auto load = [&](int c, int r2, int p2, int rb, Adds& a) {
+    const int m = kid.m[c];
+    const double* col = kid.cb[c] + (size_t)kid.cld[c] * r2;
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const int r1 = rb + 32 * u;
-          dst[u] = nullptr;
-          if (r1 < m) {
-            int p1;
-            if (r1 < nd) {
-              p1 = off + r1;
-            } else {
-              p1 = cm[r1 - nd];
-              if (p1 >= ns) p1 += nd_in;
-            }
-            dst[u] = (p1 >= p2) ? F + (p1 + (size_t)f * p2) : F + (p2 + (size_t)f * p1);
-            val[u] = col[r1];
-          }
-        }
-        double old[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) old[u] = dst[u] ? *dst[u] : 0.0;
-#pragma unroll
-        for (int u = 0; u < 4; u++)
-          if (dst[u]) *dst[u] = old[u] + val[u];
+    for (int u = 0; u < 4; u++) {
+      const int r1 = rb + 32 * u;
+      a.dst[u] = nullptr;
+      a.val[u] = 0.0;
+      if (r1 < m) {
+        const int p1 = place(c, r1);
+        a.dst[u] = (p1 >= p2) ? F + (p1 + (size_t)f * p2) : F + (p2 + (size_t)f * p1);
+        a.val[u] = col[r1];
       }
     }
-    off += nd;
+  };
+  auto first = [&](int c, Adds& a) {
+    const int r2 = rank * kW + warp;
+#pragma unroll
+    for (int u = 0; u < 4; u++) a.dst[u] = nullptr;
+    if (r2 < kid.m[c]) load(c, r2, place(c, r2), r2 + lane, a);
+  };
+  for (int q0 = kb; q0 < ke; q0 += 32) {
+    const int n = min(32, ke - q0);
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      int nd = 0;
+      if (lane < n) {
+        const int ch = p.kids[q0 + lane];
+        nd = s.ndel[ch];
+        kid.nd[lane] = nd;
+        kid.m[lane] = s.f[ch] - s.npiv[ch];
+        kid.cb[lane] = s.dpool + s.cb_off[ch];
+        kid.cld[lane] = s.cb_ld[ch];
+        kid.cm[lane] = p.cmap + p.cptr[ch];
+      }
+      int incl = nd;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+      }
+      const int base = kid.next_off;
+      if (lane < n) kid.off[lane] = base + incl - nd;
+      __syncwarp();
+      if (lane == 31) kid.next_off = base + incl;
+    }
+    __syncthreads();
+    Adds next;
+    first(0, next);
+    for (int c = 0; c < n; c++) {
+      asm_sync<CL>();
+      const Adds now = next;
+      double old[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) old[u] = now.dst[u] ? *now.dst[u] : 0.0;
+      if (c + 1 < n) first(c + 1, next);
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (now.dst[u]) *now.dst[u] = old[u] + now.val[u];
+      const int m = kid.m[c];
+      for (int r2 = rank * kW + warp; r2 < m; r2 += CL * kW) {
+        const int p2 = place(c, r2);
+        const bool again = r2 == rank * kW + warp;  // its first 128 rows are added
+        // four entries per lane pass: their loads (map, value, front) are in
+        // flight together before the read-modify-writes
+        for (int rb = r2 + lane + (again ? 128 : 0); rb < m; rb += 128) {
+          Adds a;
+          load(c, r2, p2, rb, a);
+          double o[4];
+#pragma unroll
+          for (int u = 0; u < 4; u++) o[u] = a.dst[u] ? *a.dst[u] : 0.0;
+#pragma unroll
+          for (int u = 0; u < 4; u++)
+            if (a.dst[u]) *a.dst[u] = o[u] + a.val[u];
+        }
+      }
+    }
   }
 }
 
