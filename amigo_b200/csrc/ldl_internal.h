@@ -16,7 +16,7 @@ constexpr int kWork = 8;
 
 // Kernel classes timed by the optional profiler.
 enum ProfPhase : int {
-  kPhFront = 0,     // per-level front kernels (assembly + factor in shared memory)
+  kPhFront = 0,     // fronts of one CTA (assembly + factor on chip)
   kPhBigAsm = 1,    // big-front assembly (zero, scatter, extend-add)
   kPhBigPanel = 2,  // cluster panel factorization
   kPhBigUpd = 3,    // tiled trailing update
@@ -242,7 +242,8 @@ struct FactorParams {
   int mixed;
 };
 
-// Largest front factored entirely in shared memory (fp64, ld = f | 1).
+// Largest front that one CTA factors on chip (registers, or shared memory with
+// ld = f | 1).
 constexpr int kSmemFrontMax = 144;
 constexpr int kFactorThreads = 256;
 
