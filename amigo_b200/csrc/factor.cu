@@ -49,14 +49,17 @@ __device__ __forceinline__ double warp_max(double v) {
 }
 
 // The CTA's two column barriers (used in turn), split into halves: the warp
-// that has published a column arrives and goes on, the others wait for it.
+// that has published a column arrives and goes on, the others wait for it. A
+// warp executes either as one, so its lanes come together first.
 __device__ __forceinline__ void bar_arrive(int odd) {
+  __syncwarp();
   if (odd)
     asm volatile("bar.arrive 2, %0;" ::"n"(kFactorThreads) : "memory");
   else
     asm volatile("bar.arrive 1, %0;" ::"n"(kFactorThreads) : "memory");
 }
 __device__ __forceinline__ void bar_wait(int odd) {
+  __syncwarp();
   if (odd)
     asm volatile("bar.sync 2, %0;" ::"n"(kFactorThreads) : "memory");
   else
