@@ -387,6 +387,7 @@ __global__ void __launch_bounds__(kPanelThreads)
   int kw = 0;
   int npos = 0, nneg = 0;
   double flops = 0.0;
+  cl.sync();  // every CTA has started (the partials go to all of them)
 
   {  // one panel
   kstart = k;

@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(kBcThreads)
     perm[p] = (unsigned short)p;
     ipos[p] = (unsigned short)p;
   }
-  __syncthreads();
+  cl.sync();  // every CTA has started (the exchanges write to all of them)
 
   int kw = 0;
   int npos = 0, nneg = 0;

@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(kSbThreads)
             get32(L, ldl, b * kTileR, end_of(b), b * kTileR, end_of(b), warp, lane), warp, lane);
     load_rows(b, max(end_of(b), rb) + lane, nx);
   }
-  __syncthreads();
+  cl.sync();  // every CTA has started: the partial sums go to another's memory
   for (int b = ntile - 1; b >= 0; b--) {
     const int jb = b * kTileR;
     const int je = end_of(b);
