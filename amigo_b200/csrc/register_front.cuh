@@ -89,6 +89,7 @@ struct Chain {
   int k, ncand;
   double *cur, *nx1, *nx2;  // the column at k, the next, the one after
   bool forced;  // the candidate at k is accepted as it stands
+  bool zero;    // and as a zero pivot: the other rows stay as they are
   bool moved;   // the column at k stands in cur alone (after a delay)
   int phase;    // which column barrier is next
   double thr, tol;  // a 1x1 passes with |d| >= tol and |d| >= thr max|column|
@@ -134,7 +135,7 @@ __device__ __forceinline__ void stage(double (&v)[kS][kR], Chain& h, const Front
     }
     const double d = cur[kD];
     const double absd = fabs(d);
-    const double r = (h.root && d == 0.0) ? 0.0 : 1.0 / d;
+    const double r = (h.zero || (h.root && d == 0.0)) ? 0.0 : 1.0 / d;
     if (!h.forced && !h.any) {
       // a bound of the lane's largest entry from its high word: a pivot that
       // passes against it passes (the rounded product is monotone), the full
@@ -143,6 +144,7 @@ __device__ __forceinline__ void stage(double (&v)[kS][kR], Chain& h, const Front
       if (!__all_sync(0xffffffffu, ok)) return;
     }
     h.forced = false;
+    h.zero = false;
     h.moved = false;
     const int nxt = k + 1;
     const bool more = nxt < h.ncand;
@@ -270,7 +272,7 @@ __device__ __forceinline__ Result factor_front(const Front& a, bool root, const 
   double* U = V + kLen;
   h.k = 0;
   h.ncand = a.fs;
-  h.forced = h.moved = false;
+  h.forced = h.zero = h.moved = false;
   h.phase = 0;
   h.thr = root ? kAlphaBK : prm.ustab;
   h.tol = root ? 0.0 : prm.pivot_tol;
@@ -481,6 +483,7 @@ __device__ __forceinline__ Result factor_front(const Front& a, bool root, const 
       // too, after an interchange).
       if (formed) __syncthreads();
       h.forced = true;
+      h.zero = step == kZero;
       continue;
     }
     // a 2x2 pivot: columns k and k + 1, with imax at k + 1

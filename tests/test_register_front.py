@@ -91,3 +91,24 @@ def test_candidates_and_rows(lib, f, fs, kind, ustab):
 def test_cholesky(lib, f, fs):
     out = _check(lib, _matrix("definite", f, fs, f), fs, 0, 1, 0.01, 6)
     assert out["pivots"] == out["pos"] == fs and out["moved"] == 0
+
+
+@pytest.mark.parametrize("root", [0, 1])
+@pytest.mark.parametrize("f,at", [(6, 2), (40, 0), (40, 39), (70, 33)])
+@pytest.mark.parametrize("what", ["isolated nan", "nan", "isolated inf", "inf", "nan row",
+                                  "isolated zero", "tiny"])
+def test_values_that_are_not_numbers(lib, f, at, what, root):
+    """Not-a-number, infinite and zero entries take the pivots that the plain
+    loops take (a pivot column that is zero or not a number throughout counts
+    as a zero pivot at a root, and leaves the other rows as they are)."""
+    a = _matrix("zeros", f, f, f + at)
+    if what.startswith("isolated"):
+        a[at, :] = a[:, at] = 0.0
+    value = {"nan": np.nan, "inf": np.inf, "zero": 0.0, "tiny": 1e-310}
+    if what == "nan row":
+        a[at, :] = a[:, at] = np.nan
+    else:
+        a[at, at] = value[what.split()[-1]]
+    if what == "inf":
+        a[(at + 1) % f, at] = a[at, (at + 1) % f] = -np.inf
+    _check(lib, a, f if root else f - 2, root, 0, 0.01, 2)
