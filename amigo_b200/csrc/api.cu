@@ -206,6 +206,7 @@ struct b200ldl_handle {
   std::vector<SolveRun> solve_runs;
   std::vector<int> solve_nodes;  // host copy of d_solve_nodes
   DevBuf<int> d_solve_nodes, d_parent, d_fdone, d_bdone, d_solve_ticket;
+  int wait_polls = kWaitPolls;
   int solve_epoch = 0;        // solves so far (the flags' values follow it)
   int* solve_fail = nullptr;  // pinned host memory
   Prof prof;
@@ -598,7 +599,8 @@ void run_factor_once(b200ldl_t h, const double* vals, const double* diag, bool m
   // candidates where they stand: their big fronts take the blocked panels
   // with a-posteriori tests
   FactorParams prm{h->ustab, h->pivot_tol, h->solver_type == B200LDL_CHOLESKY ? 1 : 0,
-                   (h->replanned && h->solver_type != B200LDL_CHOLESKY) ? 1 : 0, 0, 0};
+                   (h->replanned && h->solver_type != B200LDL_CHOLESKY) ? 1 : 0, 0, 0,
+                   h->wait_polls};
   prm.mixed = (prm.app && mixed) ? 1 : 0;
   h->factored_mixed = prm.mixed != 0;
   h->last_vals = vals;
@@ -712,7 +714,8 @@ void run_factor_once(b200ldl_t h, const double* vals, const double* diag, bool m
       }
       return;
     }
-    if (err[0] & 8) throw std::runtime_error("a front's children did not complete in time");
+    // (a wait given up beside another failure is that one's: factor again)
+    if (err[0] == 8) throw std::runtime_error("a front's children did not complete in time");
     if (err[0] & 4) {
       // a front went big in a level not prepared for one: every level whose
       // bound allows one is prepared
@@ -840,6 +843,7 @@ void run_solve(b200ldl_t h, int nrhs, double* x, int ldx) {
       sp.epoch = h->solve_epoch;
       sp.fail = h->d_err.ptr + 3;
       sp.host_fail = h->solve_fail;
+      sp.wait_polls = h->wait_polls;
       return sp;
     };
     for (int q = 0; q < nruns; q++) {
@@ -1457,6 +1461,13 @@ int b200ldl_solve_refine(b200ldl_t h, const double* vals, const double* diag, in
     refine_impl(h, vals, diag, nrhs, b, ldb, x, ldx, max_iter, tol, berr_out, iters_out);
     return 0;
   });
+}
+
+int b200ldl_set_wait_limit(b200ldl_t h, int polls) {
+  if (!h) return -1;
+  if (polls < 0) return fail(h, -1, "the wait limit must not be negative");
+  h->wait_polls = polls;
+  return 0;
 }
 
 int b200ldl_set_profiling(b200ldl_t h, int enable) {

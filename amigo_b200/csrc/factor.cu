@@ -556,7 +556,7 @@ __global__ void __launch_bounds__(kFactorThreads, kMax == 1 ? 4 : kMax == 2 ? 3 
         int nd = 0, fail = 0;
         for (int c = kb + lane; c < ke; c += 32) {
           const int ch = p.kids[c];
-          if (ticket && !wait_flag(s.done + ch, 1, s.err, 8)) fail = 1;
+          if (ticket && !wait_flag(s.done + ch, 1, s.err, 8, prm.wait_polls)) fail = 1;
           nd += __ldcg(s.ndel + ch);
         }
         nd = __reduce_add_sync(0xffffffffu, nd);

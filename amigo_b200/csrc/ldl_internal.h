@@ -195,18 +195,21 @@ __device__ __forceinline__ int flag_get(const int* flag) {
   return v;
 }
 
-// Polls the flag until it is at least `value`; false after kWaitPolls polls
-// (several seconds; a wait normally takes microseconds) or once *fail is set,
-// which whoever gives up sets to `code`. Both are in device memory: a read of
-// host memory in the loop would hold up the release of every flag on the SM
-// (a CTA's fence waits for the SM's loads; 20 ms instead of 1.7 for the
-// backward sweep of the 64 x 64 plane-stress system). The polls are relaxed
-// and the acquire comes once, since an acquiring load empties the SM's L1.
+// Polls the flag until it is at least `value`; false after `limit` polls or
+// once *fail is set, to which whoever gives up adds the bit `code` (the bits
+// of other failures stay in the word: they say what the host does next). Both
+// are in device memory: a read of host memory in the loop would hold up the
+// release of every flag on the SM (a CTA's fence waits for the SM's loads; 20
+// ms instead of 1.7 for the backward sweep of the 64 x 64 plane-stress
+// system). The polls are relaxed and the acquire comes once, since an
+// acquiring load empties the SM's L1. A wait normally takes microseconds;
+// kWaitPolls, the limit unless the handle has another, is several seconds.
 constexpr int kWaitPolls = 1 << 23;
-__device__ __forceinline__ bool wait_flag(const int* flag, int value, int* fail, int code) {
+__device__ __forceinline__ bool wait_flag(const int* flag, int value, int* fail, int code,
+                                          int limit) {
   for (int polls = 0; flag_get(flag) < value; polls++) {
-    if (polls > kWaitPolls) {
-      *((volatile int*)fail) = code;
+    if (polls >= limit) {
+      atomicOr(fail, code);
       return false;
     }
     if ((polls & 255) == 255 && *((volatile int*)fail) != 0) return false;
@@ -240,6 +243,7 @@ struct FactorParams {
   // mixed precision: the contribution-block tiles of the a-posteriori panels'
   // trailing updates on the tensor cores (3xTF32, FP32 accumulation)
   int mixed;
+  int wait_polls;  // limit of a wait for a child
 };
 
 // Largest front that one CTA factors on chip (registers, or shared memory with
@@ -325,6 +329,7 @@ struct SolveSpan {
   int epoch;          // number of the solve; the flags of earlier ones are smaller
   int* fail;          // device memory, set when a wait was given up
   int* host_fail;     // and host memory
+  int wait_polls;     // limit of a wait
 };
 // sweeps: 1 forward, 2 backward, 3 both in one launch
 void launch_solve(const DevPlan& p, const DevState& s, const SolveSpan& sp, int sweeps, double* x,

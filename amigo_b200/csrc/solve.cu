@@ -223,6 +223,7 @@ struct SolveArgs {
   int epoch;
   int* fail;          // set when a wait was given up
   int* host_fail;     // the same for the host to read
+  int wait_polls;     // limit of a wait
   int sweeps;         // 1: forward, 2: backward, 3: forward, then backward
   double* x;
   int ldx, nrhs, r0, nr;
@@ -325,7 +326,7 @@ __device__ __forceinline__ bool forward_node(const DevPlan& p, const DevState& s
   if (a.ticket && warp == 0) {
     bool ok = true;
     for (int c = kb + lane; c < ke; c += 32)
-      ok = wait_flag(a.fdone + p.kids[c], 2 * a.epoch, a.fail, 1) && ok;
+      ok = wait_flag(a.fdone + p.kids[c], 2 * a.epoch, a.fail, 1, a.wait_polls) && ok;
     ok = __all_sync(0xffffffffu, ok);
     if (lane == 0 && !ok) *sh_fail = 1;
   }
@@ -514,7 +515,8 @@ __device__ __forceinline__ bool backward_node(const DevPlan& p, const DevState& 
     }
     if (lane == 0) bst[nb] = npiv;
   }
-  if (a.sweeps == 3 && tid == 32 && !wait_flag(a.fdone + node, 2 * a.epoch + 1, a.fail, 1))
+  if (a.sweeps == 3 && tid == 32 &&
+      !wait_flag(a.fdone + node, 2 * a.epoch + 1, a.fail, 1, a.wait_polls))
     *sh_fail = 1;  // the own forward solution
   __syncthreads();
   if (*sh_fail) return false;
@@ -541,7 +543,8 @@ __device__ __forceinline__ bool backward_node(const DevPlan& p, const DevState& 
   gather(0, npiv);
   if (a.ticket && tid == 0) {
     const int par = a.parent[node];
-    if (par >= 0 && !wait_flag(a.bdone + par, 2 * a.epoch + 1, a.fail, 1)) *sh_fail = 1;
+    if (par >= 0 && !wait_flag(a.bdone + par, 2 * a.epoch + 1, a.fail, 1, a.wait_polls))
+      *sh_fail = 1;
   }
   __syncthreads();
   if (*sh_fail) return false;
@@ -670,6 +673,7 @@ void launch_solve(const DevPlan& p, const DevState& s, const SolveSpan& sp, int 
   a.epoch = sp.epoch;
   a.fail = sp.fail;
   a.host_fail = sp.host_fail;
+  a.wait_polls = sp.wait_polls;
   a.sweeps = sweeps;
   a.x = x;
   a.ldx = ldx;

@@ -492,6 +492,12 @@ class SparseLDL:
     PHASES =("fronts", "big_assembly", "big_panel", "big_update", "solve_forward",
               "solve_backward", "cluster_fronts")
 
+    def set_wait_limit(self, polls: int):
+        """Polls after which a thread block gives up waiting for another's
+        front; the call then raises."""
+        if self._lib.b200ldl_set_wait_limit(self._h, polls) != 0:
+            raise ValueError(self._lib.b200ldl_last_error(self._h).decode())
+
     def set_profiling(self, on: bool):
         self._lib.b200ldl_set_profiling(self._h, 1 if on else 0)
 

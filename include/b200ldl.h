@@ -254,6 +254,14 @@ int b200ldl_reuse_pivot_order(b200ldl_t h);
  * delayed pivots summed over supernodes, stats[5] = number of levels. */
 int b200ldl_stats(b200ldl_t h, double* stats, int nstats);
 
+/* Limit of the waits inside a launch (no counterpart in the reference). A
+ * launch that covers several levels of the tree has its thread blocks wait
+ * for one another's fronts; a wait that has polled `polls` times is given up,
+ * the kernel ends, and the call returns status -4 (the factor or the solution
+ * is then undefined, the handle stays usable). The default is 2^23 polls,
+ * seconds where a wait takes microseconds. */
+int b200ldl_set_wait_limit(b200ldl_t h, int polls);
+
 /* Profiling (no counterpart in the reference, which has no GPU timers):
  * when enabled, CUDA events on the handle's stream time each kernel class.
  * b200ldl_profile writes, for each class p in {fronts, big-front assembly,
