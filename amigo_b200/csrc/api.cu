@@ -207,7 +207,7 @@ struct b200ldl_handle {
   std::vector<int> solve_nodes;  // host copy of d_solve_nodes
   DevBuf<int> d_solve_nodes, d_parent, d_fdone, d_bdone, d_solve_ticket;
   int wait_polls = kWaitPolls;
-  int solve_epoch = 0;        // solves so far (the flags' values follow it)
+  int solve_epoch = 0;        // solves since the flags were cleared (their values follow it)
   int* solve_fail = nullptr;  // pinned host memory
   Prof prof;
   double flops4[kWork] = {};
@@ -822,6 +822,14 @@ void run_solve(b200ldl_t h, int nrhs, double* x, int ldx) {
   const bool both = nruns == 1 && h->solve_runs[0].big_count == 0;
   for (int r0 = 0; r0 < nrhs; r0 += chunk) {
     const int nr = std::min(chunk, nrhs - r0);
+    // the flags' values grow with the solves: they start over long before
+    // they leave the range of an int (two small memsets in 4,096 solves)
+    constexpr int kEpochs = 4096;
+    if (h->solve_epoch >= kEpochs) {
+      CK(cudaMemsetAsync(h->d_fdone.ptr, 0, h->d_fdone.count * sizeof(int), h->stream));
+      CK(cudaMemsetAsync(h->d_bdone.ptr, 0, h->d_bdone.count * sizeof(int), h->stream));
+      h->solve_epoch = 0;
+    }
     h->solve_epoch++;
     CK(cudaMemsetAsync(h->d_solve_ticket.ptr, 0, 2 * std::max(1, nruns) * sizeof(int),
                        h->stream));

@@ -47,7 +47,8 @@ constexpr int kMaxRhs = kSWarps;  // right-hand sides per launch: a warp each
 // Progress of a supernode in the solve numbered `epoch`: its flags hold
 // 2 epoch once the update vector is written, 2 epoch + 1 once the forward
 // solution is, and, in the backward sweep's array, 2 epoch + 1 once the final
-// solution is. They only grow, so that a solve needs no clearing.
+// solution is. They grow from solve to solve, so that a solve needs no
+// clearing (the host clears them and starts over after some thousand solves).
 
 // end of the pivot block starting at jb: at most 32 pivots, and 2x2 pairs
 // never straddle two blocks
