@@ -126,8 +126,7 @@ struct b200ldl_handle {
   const double* last_vals = nullptr;
   // element-block source of the factorization in progress (nullptr: CSR
   // values)
-  const long long* asm_ptr = nullptr;
-  const long long* asm_src = nullptr;
+  AsmPlan asm_plan;
   const double* asm_blocks = nullptr;
   const double* last_diag = nullptr;
   int last_iters = 0;
@@ -560,8 +559,7 @@ void bind_state(b200ldl_t h) {
   st.class_list = h->d_class_list.ptr;
   for (int c = 0; c < 5; c++) st.cf_limit[c] = cluster_front_limit(c);
   st.partner = h->replanned ? h->d_partner.ptr : nullptr;
-  st.asm_ptr = h->asm_ptr;
-  st.asm_src = h->asm_src;
+  st.asm_plan = h->asm_plan;
   st.asm_blocks = h->asm_blocks;
 }
 
@@ -1126,8 +1124,8 @@ int b200ldl_factor_elements(b200ldl_t h, b200ldl_assembly_t a, const double* blo
                             const double* diag) {
   return guarded(h, [&]() {
     int an = 0, annz = 0;
-    const long long *aptr = nullptr, *asrc = nullptr;
-    if (!a || assembly_device_plan(a, &an, &annz, &aptr, &asrc) != 0)
+    AsmPlan plan;
+    if (!a || assembly_device_plan(a, &an, &annz, &plan) != 0)
       return fail(h, -1, "no assembly plan");
     if (an != h->n || annz != h->nnz)
       return fail(h, -1,
@@ -1142,14 +1140,11 @@ int b200ldl_factor_elements(b200ldl_t h, b200ldl_assembly_t a, const double* blo
     struct Source {
       b200ldl_t h;
       ~Source() {
-        h->asm_ptr = h->asm_src = nullptr;
-        h->asm_blocks = nullptr;
-        h->st.asm_ptr = h->st.asm_src = nullptr;
-        h->st.asm_blocks = nullptr;
+        h->asm_plan = h->st.asm_plan = AsmPlan{};
+        h->asm_blocks = h->st.asm_blocks = nullptr;
       }
     } source{h};
-    h->asm_ptr = h->st.asm_ptr = aptr;
-    h->asm_src = h->st.asm_src = asrc;
+    h->asm_plan = h->st.asm_plan = plan;
     h->asm_blocks = h->st.asm_blocks = blocks;
     h->factored = false;
     h->fmax = 0;

@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <cstdarg>
 #include <cstdio>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -84,9 +85,10 @@ __global__ void __launch_bounds__(256)
 template <typename T>
 struct DevArr {
   T* ptr = nullptr;
-  size_t count = 0;
-  ~DevArr() {
+  ~DevArr() { release(); }
+  void release() {
     if (ptr) cudaFree(ptr);
+    ptr = nullptr;
   }
 };
 
@@ -101,8 +103,10 @@ struct b200ldl_assembly {
   std::vector<int> ptr32, src32;
   bool narrow = false;
   long long kept() const { return narrow ? (long long)src32.size() : (long long)src.size(); }
-  DevArr<long long> d_ptr, d_src;  // for factorizations from element blocks
-  DevArr<int> d_ptr32, d_src32;    // for the gather, where the plan fits
+  // and the device copy, one of the pairs, complete once `uploaded` is set
+  DevArr<long long> d_ptr, d_src;
+  DevArr<int> d_ptr32, d_src32;
+  mutable std::mutex mu;  // of the upload
   bool uploaded = false;
   std::string last_error;
 };
@@ -131,17 +135,31 @@ inline long long find_entry(const int* rowp, const int* cols, int row, int col) 
 
 template <typename T>
 cudaError_t to_device(DevArr<T>& d, const std::vector<T>& h) {
+  d.release();
   cudaError_t e = cudaMalloc(&d.ptr, std::max<size_t>(1, h.size()) * sizeof(T));
+  if (e != cudaSuccess) d.ptr = nullptr;
   if (e == cudaSuccess && !h.empty())
     e = cudaMemcpy(d.ptr, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice);
   return e;
 }
 
+// Threads may share a plan: the first to come uploads it, and it counts as
+// uploaded once both copies have arrived (the copies' stream does not order
+// the streams that read them).
 int upload(b200ldl_assembly* a) {
+  std::lock_guard<std::mutex> lock(a->mu);
   if (a->uploaded) return 0;
   cudaError_t e = a->narrow ? to_device(a->d_ptr32, a->ptr32) : to_device(a->d_ptr, a->ptr);
   if (e == cudaSuccess) e = a->narrow ? to_device(a->d_src32, a->src32) : to_device(a->d_src, a->src);
-  if (e != cudaSuccess) return afail(a, -3, "CUDA error: %s", cudaGetErrorString(e));
+  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+  if (e != cudaSuccess) {
+    a->d_ptr32.release();
+    a->d_src32.release();
+    a->d_ptr.release();
+    a->d_src.release();
+    cudaGetLastError();  // reported here, not by the thread's next launch
+    return afail(a, -3, "CUDA error: %s", cudaGetErrorString(e));
+  }
   a->uploaded = true;
   return 0;
 }
@@ -269,19 +287,13 @@ void b200ldl_assembly_destroy(b200ldl_assembly_t a) { delete a; }
 
 namespace b200ldl {
 
-int assembly_device_plan(::b200ldl_assembly* a, int* n, int* nnz, const long long** ptr,
-                         const long long** src) {
-  if (!a || !a->uploaded) return -1;
-  if (!a->d_ptr.ptr) {
-    // the fronts' scattered reads take 64-bit indices
-    const std::vector<long long> p(a->ptr32.begin(), a->ptr32.end());
-    const std::vector<long long> q(a->src32.begin(), a->src32.end());
-    if (to_device(a->d_src, q) != cudaSuccess || to_device(a->d_ptr, p) != cudaSuccess) return -1;
-  }
+int assembly_device_plan(const ::b200ldl_assembly* a, int* n, int* nnz, AsmPlan* plan) {
+  if (!a) return -1;
+  std::lock_guard<std::mutex> lock(a->mu);
+  if (!a->uploaded) return -1;
   *n = a->n;
   *nnz = a->nnz;
-  *ptr = a->d_ptr.ptr;
-  *src = a->d_src.ptr;
+  *plan = AsmPlan{a->d_ptr32.ptr, a->d_src32.ptr, a->d_ptr.ptr, a->d_src.ptr};
   return 0;
 }
 

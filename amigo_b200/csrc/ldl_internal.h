@@ -82,6 +82,13 @@ struct Prof {
   }
 };
 
+// The device copy of an assembly plan: 32-bit indices where they fit, else
+// 64-bit ones (the other pair is null).
+struct AsmPlan {
+  const int *ptr32 = nullptr, *src32 = nullptr;
+  const long long *ptr = nullptr, *src = nullptr;
+};
+
 // Immutable per-pattern data uploaded once after the symbolic phase. All
 // arrays are indexed by supernode id (the reference's node numbering) unless
 // stated otherwise.
@@ -176,10 +183,9 @@ struct DevState {
   const int* partner;
   // factorization from element Hessian blocks (b200ldl_factor_elements): the
   // CSR value of entry e is the sum, from zero in order, of
-  // asm_blocks[asm_src[q]] for q in [asm_ptr[e], asm_ptr[e + 1]); nullptr
+  // asm_blocks[src[q]] for q in [ptr[e], ptr[e + 1]); asm_blocks is nullptr
   // when the factorization reads CSR values
-  const long long* asm_ptr;
-  const long long* asm_src;
+  AsmPlan asm_plan;
   const double* asm_blocks;
 };
 
@@ -224,9 +230,15 @@ __device__ __forceinline__ bool wait_flag(const int* flag, int value, int* fail,
 __device__ __forceinline__ double csr_value(const DevState& s, const double* __restrict__ vals,
                                             long long e) {
   if (!s.asm_blocks) return vals[e];
+  const AsmPlan& a = s.asm_plan;
   double v = 0.0;
-  const long long q1 = s.asm_ptr[e + 1];
-  for (long long q = s.asm_ptr[e]; q < q1; q++) v += s.asm_blocks[s.asm_src[q]];
+  if (a.ptr32) {
+    const int q1 = a.ptr32[e + 1];
+    for (int q = a.ptr32[e]; q < q1; q++) v += s.asm_blocks[a.src32[q]];
+  } else {
+    const long long q1 = a.ptr[e + 1];
+    for (long long q = a.ptr[e]; q < q1; q++) v += s.asm_blocks[a.src[q]];
+  }
   return v;
 }
 
@@ -371,9 +383,9 @@ void launch_copy_cols(int n, int nr, const double* src, int lds, double* dst, in
 void launch_perturb_diag(int n, const double* diag, const unsigned char* cls, double dx,
                          double dc, double* out, cudaStream_t st);
 
-// The device copy of an assembly plan (assembly.cu): its pattern's size and
-// the per-CSR-entry contribution lists. Returns 0, or -1 without a plan.
-int assembly_device_plan(::b200ldl_assembly* a, int* n, int* nnz, const long long** ptr,
-                         const long long** src);
+// The device copy of an assembly plan (assembly.cu) and its pattern's size.
+// Returns 0, or -1 before the plan is on the device. Changes nothing: handles
+// driven by several threads may share a plan.
+int assembly_device_plan(const ::b200ldl_assembly* a, int* n, int* nnz, AsmPlan* plan);
 
 }  // namespace b200ldl
