@@ -43,6 +43,16 @@ namespace {
 // entry at a time 62, four 64).
 constexpr int kPer = 2;
 
+// 32-bit indices take a plan whose contributions b, b + 1 and b + 2 of an
+// entry that begins at b can be named, also where it has none and begins at
+// the end of the list
+constexpr bool fits_32(long long values, long long contributions) {
+  return values <= 2147483647LL && contributions <= 2147483647LL - 2;
+}
+static_assert(fits_32(2147483647LL, 2147483645LL) && !fits_32(1, 2147483646LL) &&
+                  !fits_32(1, 2147483647LL) && !fits_32(2147483648LL, 1),
+              "the last entry's b + 2 is an int");
+
 template <typename Index>
 __global__ void __launch_bounds__(256)
     csr_gather_kernel(int nnz, const Index* __restrict__ ptr, const Index* __restrict__ src,
@@ -223,7 +233,7 @@ int b200ldl_assembly_create(b200ldl_assembly_t* out, int n, const int* rowp, con
     if (pass == 0) {
       for (int p = 0; p < a->nnz; p++) cnt[p + 1] += cnt[p];
       a->ptr = cnt;
-      a->narrow = a->nvals <= 2147483647LL && cnt[a->nnz] <= 2147483647LL;
+      a->narrow = fits_32(a->nvals, cnt[a->nnz]);
       if (a->narrow) {
         a->ptr32.assign(a->ptr.begin(), a->ptr.end());
         std::vector<long long>().swap(a->ptr);
