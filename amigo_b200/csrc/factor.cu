@@ -587,12 +587,16 @@ __global__ void __launch_bounds__(kFactorThreads, kMax == 1 ? 4 : kMax == 2 ? 3 
       fr.fv = reinterpret_cast<int*>(fr.vec + 5 * vec_len(f));
       fr.orig = fr.fv + f;
       pos = reinterpret_cast<int*>(fr.vec);
+      // a thread per own variable for the diagonal: two dependent loads each
+      for (int t = tid; t < ns; t += kFactorThreads) {
+        const int v = p.node_to_var[v0 + t];
+        fr.fv[t] = v;
+        fr.F[t + fr.ld * t] = 0.0 + (diag ? diag[v] : 0.0);
+      }
       for (int j = warp; j < f; j += kWarps) {
         double* col = fr.F + fr.ld * j;
-        const double dj = (diag && j < ns) ? diag[p.node_to_var[v0 + j]] : 0.0;
-        for (int i = j + lane; i < f; i += 32) col[i] = (i == j) ? 0.0 + dj : 0.0;
+        for (int i = j + lane + (j < ns && lane == 0 ? 32 : 0); i < f; i += 32) col[i] = 0.0;
       }
-      for (int t = tid; t < ns; t += kFactorThreads) fr.fv[t] = p.node_to_var[v0 + t];
       for (int t = tid; t < nc; t += kFactorThreads) fr.fv[fs + t] = p.contrib_rows[c0 + t];
       for (int t = tid; t < f; t += kFactorThreads) fr.orig[t] = t;
       __syncthreads();
@@ -754,7 +758,10 @@ __global__ void __launch_bounds__(kFactorThreads, kMax == 1 ? 4 : kMax == 2 ? 3 
     }
     __syncthreads();
     if (tid == 0) {
-      flag_set(s.done + node, 1);
+      if (ticket)
+        flag_set(s.done + node, 1);
+      else
+        s.done[node] = 1;  // for the launches that follow
       s.u_off[node] = (long long)atomicAdd(s.used + 2, (unsigned long long)m);
       if (!prm.cholesky) {
         atomicAdd(s.inertia, o.npos);
