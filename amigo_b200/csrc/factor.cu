@@ -9,8 +9,8 @@
 // factor columns, its final front-variable order and its contribution block.
 //
 // Fronts up to kSmemFrontMax are assembled in shared memory and factored in
-// registers (factor_front); larger ones are registered for the big-front
-// kernels.
+// registers (factor_front) or where they stand (general_front); larger ones
+// are registered for the big-front kernels.
 #include <climits>
 
 #include "ldl_internal.h"
@@ -114,13 +114,19 @@ __device__ void symm_swap(double* F, int ld, int f, int a, int b, int* fv, int* 
   }
 }
 
-// The same factorization in shared memory, for the fronts of more than 96
-// rows of a structure that still delays candidates through its fronts (dozens
-// per front): a delay moves its two rows and columns in shared memory in one
-// pass of the CTA, while the register front above forms and replaces them
-// slot by slot, several thousand cycles a delay at 18 slots of 5 chunks
-// (64 x 64 plane stress, first factorization: 95.6 ms with this one, 97.2
-// with registers throughout).
+// The same factorization in shared memory, with the same bits: the one for
+// fronts of more than 96 rows on a level with a launch of its own, unless the
+// structure was re-planned from a pivot record. Those are the levels beside
+// big fronts (and all levels of a first factorization, whose sizes are not
+// known yet). Where a tree has such levels without a record, its fronts delay
+// candidates by the dozen, and a delay moves two rows and columns in one pass
+// of the CTA here, while the register fronts form and replace them slot by
+// slot, several thousand cycles a delay at 18 slots of 5 chunks: plane stress
+// 64 x 64 in the first order, small fronts 7.1 ms of the factorization's 83.8
+// with this one, 8.7 of 85.5 with registers throughout (24 x 24: 14.3 and
+// 14.9 ms). Levels that share a launch have registers: optimal control with
+// 48 states, N = 40, 8.7 ms against 13.4 with this one, 64 systems of N = 20
+// of them, 530 delays each, 4.5 against 6.8.
 template <typename Write, typename Store>
 __device__ __forceinline__ Result general_front(const Front& a, bool root, const FactorParams& prm,
                                                Write write, Store store) {
@@ -222,7 +228,7 @@ __device__ __forceinline__ Result general_front(const Front& a, bool root, const
           step = kOne;
           kpiv = imax;
         } else {
-          const double det = fabs(wkk * wii - wik * wik);
+          const double det = fabs(two_products(wkk, wii, -wik, wik));
           step = kDelay;
           if (det >= prm.pivot_tol) {
             const double delta = det / fmax(abswii + abswik, abswkk + abswik);
@@ -259,8 +265,8 @@ __device__ __forceinline__ Result general_front(const Front& a, bool root, const
       for (int i = pc + 2 + tid; i < f; i += blockDim.x) {
         const double a = c0[i];
         const double b = c1[i];
-        c0[i] = a * pd0 + b * pd1;
-        c1[i] = a * pd1 + b * pd2;
+        c0[i] = two_products(a, pd0, b, pd1);
+        c1[i] = two_products(a, pd1, b, pd2);
       }
     }
 
@@ -277,7 +283,7 @@ __device__ __forceinline__ Result general_front(const Front& a, bool root, const
           double bv = -1.0, cm = 0.0;
           int bi = INT_MAX;
           for (int i = j + lane; i < f; i += 32) {
-            const double v = colj[i] - colk[i] * lj;
+            const double v = fma(-colk[i], lj, colj[i]);
             colj[i] = v;
             if (i > j) {
               const double a = fabs(v);
@@ -294,7 +300,7 @@ __device__ __forceinline__ Result general_front(const Front& a, bool root, const
             st_m = cm;
           }
         } else {
-          for (int i = j + lane; i < f; i += 32) colj[i] -= colk[i] * lj;
+          for (int i = j + lane; i < f; i += 32) colj[i] = fma(-colk[i], lj, colj[i]);
         }
       }
       if (tid == 0) {
@@ -313,20 +319,20 @@ __device__ __forceinline__ Result general_front(const Front& a, bool root, const
       const double d11 = colk[k];
       const double d21 = colk[k + 1];
       const double d22 = colk1[k + 1];
-      const double det = d11 * d22 - d21 * d21;
+      const double det = two_products(d11, d22, -d21, d21);
       const double detinv = 1.0 / det;
       const double i00 = d22 * detinv, i01 = -d21 * detinv, i11 = d11 * detinv;
       for (int j = k + 2 + warp; j < f; j += kWarps) {
         const double a = colk[j];
         const double b = colk1[j];
-        const double l0 = a * i00 + b * i01;
-        const double l1 = a * i01 + b * i11;
+        const double l0 = two_products(a, i00, b, i01);
+        const double l1 = two_products(a, i01, b, i11);
         double* colj = F + (size_t)ld * j;
         if (j == nxt && want_stats) {
           double bv = -1.0, cm = 0.0;
           int bi = INT_MAX;
           for (int i = j + lane; i < f; i += 32) {
-            const double v = colj[i] - (colk[i] * l0 + colk1[i] * l1);
+            const double v = colj[i] - two_products(colk[i], l0, colk1[i], l1);
             colj[i] = v;
             if (i > j) {
               const double aa = fabs(v);
@@ -343,7 +349,8 @@ __device__ __forceinline__ Result general_front(const Front& a, bool root, const
             st_m = cm;
           }
         } else {
-          for (int i = j + lane; i < f; i += 32) colj[i] -= colk[i] * l0 + colk1[i] * l1;
+          for (int i = j + lane; i < f; i += 32)
+            colj[i] -= two_products(colk[i], l0, colk1[i], l1);
         }
       }
       if (tid == 0) {
@@ -382,8 +389,8 @@ __device__ __forceinline__ Result general_front(const Front& a, bool root, const
     for (int i = pc + 2 + tid; i < f; i += blockDim.x) {
       const double a = c0[i];
       const double b = c1[i];
-      c0[i] = a * pd0 + b * pd1;
-      c1[i] = a * pd1 + b * pd2;
+      c0[i] = two_products(a, pd0, b, pd1);
+      c1[i] = two_products(a, pd1, b, pd2);
     }
   }
   __syncthreads();
@@ -801,6 +808,7 @@ void launch_factor_level(const DevPlan& p, const DevState& s, const int* nodes, 
                          const FactorParams& prm, cudaStream_t stream, const double* vals,
                          const double* diag) {
   if (count <= 0) return;
+  // above 96 rows: see general_front
   auto* kernel = fmax <= 32   ? factor_level_kernel<1>
                  : fmax <= 64 ? factor_level_kernel<2>
                  : fmax <= 96 ? factor_level_kernel<3>

@@ -60,6 +60,12 @@ __device__ __forceinline__ void bar_wait(int odd) {
 }
 #endif
 
+// a b + c d with its roundings fixed. The products of the 2x2 pivots are formed
+// in several places and by two algorithms, which have to give the same bits.
+__device__ __forceinline__ double two_products(double a, double b, double c, double d) {
+  return fma(a, b, __dmul_rn(c, d));
+}
+
 // The front of one CTA: assembled in shared memory, factored in registers.
 struct Front {
   double* F;     // [f][ld], column-major lower triangle, then the factor columns
@@ -437,7 +443,7 @@ __device__ __forceinline__ Result factor_front(const Front& a, bool root, const 
         step = kOne;
         kpiv = imax;
       } else {
-        const double det = fabs(fma(d, wii, -__dmul_rn(wik, wik)));
+        const double det = fabs(two_products(d, wii, -wik, wik));
         step = kDelay;
         if (det >= prm.pivot_tol) {
           const double delta = det / fmax(abswii + abswik, absd + abswik);
@@ -498,7 +504,7 @@ __device__ __forceinline__ Result factor_front(const Front& a, bool root, const 
     const double d11 = d;
     const double d21 = cur[q];
     const double d22 = V[kD];
-    const double det = fma(d11, d22, -__dmul_rn(d21, d21));
+    const double det = two_products(d11, d22, -d21, d21);
     const double detinv = 1.0 / det;
     const double i00 = d22 * detinv, i01 = -d21 * detinv, i11 = d11 * detinv;
     // the two columns' entries in row i (row q holds what stood at k + 1) and
@@ -506,8 +512,8 @@ __device__ __forceinline__ Result factor_front(const Front& a, bool root, const 
     // places and has to come out the same
     auto at0 = [&](int i) { return cur[i == q ? k + 1 : i]; };
     auto at1 = [&](int i) { return V[i == q ? k + 1 : i]; };
-    auto l0 = [&](double x, double y) { return fma(x, i00, __dmul_rn(y, i01)); };
-    auto l1 = [&](double x, double y) { return fma(x, i01, __dmul_rn(y, i11)); };
+    auto l0 = [&](double x, double y) { return two_products(x, i00, y, i01); };
+    auto l1 = [&](double x, double y) { return two_products(x, i01, y, i11); };
     double w0[kR], w1[kR];
 #pragma unroll
     for (int c = 0; c < kR; c++) {
@@ -538,7 +544,7 @@ __device__ __forceinline__ Result factor_front(const Front& a, bool root, const 
       const double x = on ? at0(j) : 0.0, y = on ? at1(j) : 0.0;
       const double a0 = l0(x, y), a1 = l1(x, y);
 #pragma unroll
-      for (int c = s / 4; c < kR; c++) v[s][c] -= fma(w0[c], a0, __dmul_rn(w1[c], a1));
+      for (int c = s / 4; c < kR; c++) v[s][c] -= two_products(w0[c], a0, w1[c], a1);
     }
     if (tid == 0) {
       a.fv[k] = -(a.fv[k] + 1);
