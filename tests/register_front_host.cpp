@@ -159,6 +159,11 @@ static double __hiloint2double(int hi, int lo) {
 static long long __double_as_longlong(double d) { return (long long)bits(d); }
 static double __longlong_as_double(long long u) { return bits((uint64_t)u); }
 static double __dmul_rn(double a, double b) { return a * b; }
+static int atomicOr(int* p, int v) {  // named by the header, not used here
+  const int old = *p;
+  *p |= v;
+  return old;
+}
 static void __syncwarp() { sim::exchange(0); }
 static void __syncthreads() { sim::wait(0); }
 static int __all_sync(unsigned, int v) {
