@@ -14,6 +14,23 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "slow: long-running CPU test")
 
 
+def pytest_collection_modifyitems(items):
+    """Where the compiled reference was not built, the modules that use it run
+    after the others: a run that stops at the first failure then stops at a
+    test that lacks its oracle only when the rest has run."""
+    from oracle import ref
+
+    if ref.available():
+        return
+    uses = {}
+    for item in items:
+        path = str(item.path)
+        if path not in uses:
+            text = open(path).read()
+            uses[path] = "oracle" in text or '"--impl", "reference"' in text
+    items.sort(key=lambda item: uses[str(item.path)])
+
+
 @pytest.fixture(scope="session")
 def golden():
     return np.load(os.path.join(ROOT, "tests", "golden", "ldl_cases.npz"))
