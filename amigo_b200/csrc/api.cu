@@ -46,6 +46,7 @@ struct DevBuf {
     else ptr = nullptr;
     return e;
   }
+  // (uploads_arrived() before another stream's work reads it)
   cudaError_t upload(const std::vector<T>& h) {
     cudaError_t e = alloc(h.size());
     if (e != cudaSuccess) return e;
@@ -53,6 +54,10 @@ struct DevBuf {
     return e;
   }
 };
+
+// A copy from pageable memory may return before its last part has arrived, and
+// it is in the default stream, which does not order a non-blocking one.
+cudaError_t uploads_arrived() { return cudaStreamSynchronize(nullptr); }
 
 struct CudaError : std::runtime_error {
   cudaError_t code;
@@ -486,6 +491,8 @@ void upload_plan(b200ldl_t h) {
   CK(h->d_rowp.upload(h->h_rowp));
   CK(h->d_cols.upload(h->h_cols));
   if (h->replanned) CK(h->d_partner.upload(h->partner));
+  CK(h->d_parent.upload(s.parent));
+  CK(uploads_arrived());
 
   DevPlan& p = h->plan;
   p.n = s.n;
@@ -516,7 +523,6 @@ void upload_plan(b200ldl_t h) {
   CK(h->d_cb_off.alloc(nn));
   CK(h->d_u_off.alloc(nn));
   CK(h->d_done.alloc(nn));
-  CK(h->d_parent.upload(s.parent));
   CK(h->d_fdone.alloc(nn));
   CK(h->d_bdone.alloc(nn));
   CK(cudaMemsetAsync(h->d_fdone.ptr, 0, h->d_fdone.count * sizeof(int), h->stream));
@@ -689,7 +695,10 @@ void run_factor_once(b200ldl_t h, const double* vals, const double* diag, bool m
     h->prof.collect();
     if (err[0] == 0) {
       if (h->nsys > 1 && h->solver_type != B200LDL_CHOLESKY) {
-        if (h->d_node_sys.count < h->node_sys.size()) CK(h->d_node_sys.upload(h->node_sys));
+        if (h->d_node_sys.count < h->node_sys.size()) {
+          CK(h->d_node_sys.upload(h->node_sys));
+          CK(uploads_arrived());
+        }
         if (h->d_sys_inertia.count < (size_t)2 * h->nsys) CK(h->d_sys_inertia.alloc(2 * h->nsys));
         CK(cudaMemsetAsync(h->d_sys_inertia.ptr, 0, 2 * h->nsys * sizeof(int), h->stream));
         launch_system_inertia(h->st, h->d_node_sys.ptr, h->sym.num_nodes, h->d_sys_inertia.ptr,
@@ -763,7 +772,8 @@ void level_fronts(b200ldl_t h) {
   CK(cudaMemcpy(f.data(), h->d_f.ptr, nn * sizeof(int), cudaMemcpyDeviceToHost));
   h->level_fmax.assign(h->num_levels, 1);
   h->solve_runs.clear();
-  h->solve_nodes.clear();
+  std::vector<int> nodes;
+  nodes.reserve(nn);
   int m = 1;
   b200ldl_handle::SolveRun run;
   std::vector<int> big;
@@ -779,7 +789,7 @@ void level_fronts(b200ldl_t h) {
         run.big_fmax = std::max(run.big_fmax, fn);
         continue;
       }
-      h->solve_nodes.push_back(node);
+      nodes.push_back(node);
       run.fmax = std::max(run.fmax, fn);
       width++;
     }
@@ -788,20 +798,24 @@ void level_fronts(b200ldl_t h) {
     run.levels += width > 0;
     m = std::max(m, run.fmax);
     if (!big.empty() || l + 1 == h->num_levels) {
-      h->solve_nodes.insert(h->solve_nodes.end(), big.begin(), big.end());
+      nodes.insert(nodes.end(), big.begin(), big.end());
       run.big_count = (int)big.size();
       h->solve_runs.push_back(run);
       run = b200ldl_handle::SolveRun();
-      run.first = (int)h->solve_nodes.size();
+      run.first = (int)nodes.size();
     }
   }
   const size_t tickets = 2 * std::max<size_t>(1, h->solve_runs.size());
   if (h->d_solve_ticket.count < tickets) CK(h->d_solve_ticket.alloc(tickets));
-  if (h->d_solve_nodes.count < h->solve_nodes.size())
-    CK(h->d_solve_nodes.alloc(h->solve_nodes.size()));
-  if (!h->solve_nodes.empty())
-    CK(cudaMemcpy(h->d_solve_nodes.ptr, h->solve_nodes.data(),
-                  h->solve_nodes.size() * sizeof(int), cudaMemcpyHostToDevice));
+  // (mostly the same from one factorization to the next)
+  if (nodes != h->solve_nodes) {
+    h->solve_nodes.clear();
+    if (h->d_solve_nodes.count < nodes.size()) CK(h->d_solve_nodes.alloc(nodes.size()));
+    CK(cudaMemcpyAsync(h->d_solve_nodes.ptr, nodes.data(), nodes.size() * sizeof(int),
+                       cudaMemcpyHostToDevice, h->stream));
+    CK(cudaStreamSynchronize(h->stream));  // the solves may run in another stream
+    h->solve_nodes = std::move(nodes);
+  }
   h->fmax = m;  // largest front left to the one-CTA kernels
 }
 
