@@ -73,15 +73,17 @@ struct CudaError : std::runtime_error {
 
 // Words of pinned host memory that kernels write a failure to, one per handle
 // that has solved. A pinned allocation takes longer than a small solve, so
-// they are handed out of pages that the process keeps (one page serves 1024
-// handles at a time).
+// they are handed out of pages that the process keeps: one page serves 1024
+// handles at a time, so the pages follow the most handles alive at once.
 class HostWords {
  public:
   int* take() {
     std::lock_guard<std::mutex> lock(mu_);
     if (free_.empty()) {
+      free_.reserve(words_ + kPerPage);  // give() never allocates
       int* page = nullptr;
       CK(cudaHostAlloc(&page, kPerPage * sizeof(int), cudaHostAllocPortable));
+      words_ += kPerPage;
       for (int i = 0; i < kPerPage; i++) free_.push_back(page + i);
     }
     int* w = free_.back();
@@ -97,6 +99,7 @@ class HostWords {
  private:
   static constexpr int kPerPage = 1024;
   std::mutex mu_;
+  size_t words_ = 0;
   std::vector<int*> free_;
 };
 
@@ -105,9 +108,19 @@ HostWords& host_words() {
   return *words;
 }
 
+struct FailWord {
+  int* ptr = nullptr;
+  ~FailWord() {
+    if (ptr) host_words().give(ptr);
+  }
+};
+
 }  // namespace
 
 struct b200ldl_handle {
+  // given back last, after the device buffers: freeing those waits for kernels
+  // that a failed call left behind, which may still write to it
+  FailWord solve_fail;
   int n = 0, nnz = 0;
   int solver_type = B200LDL_LDL;
   double ustab = 0.01, pivot_tol = 1e-14, delay_growth = 2.0;
@@ -212,13 +225,9 @@ struct b200ldl_handle {
   DevBuf<int> d_solve_nodes, d_parent, d_fdone, d_bdone, d_solve_ticket;
   int wait_polls = kWaitPolls;
   int solve_epoch = 0;        // solves since the flags were cleared (their values follow it)
-  int* solve_fail = nullptr;  // pinned host memory
   Prof prof;
   double flops4[kWork] = {};
   double sum_delayed = 0.0;
-  ~b200ldl_handle() {
-    if (solve_fail) host_words().give(solve_fail);
-  }
 };
 
 namespace {
@@ -527,7 +536,7 @@ void upload_plan(b200ldl_t h) {
   CK(h->d_bdone.alloc(nn));
   CK(cudaMemsetAsync(h->d_fdone.ptr, 0, h->d_fdone.count * sizeof(int), h->stream));
   CK(cudaMemsetAsync(h->d_bdone.ptr, 0, h->d_bdone.count * sizeof(int), h->stream));
-  if (!h->solve_fail) h->solve_fail = host_words().take();
+  if (!h->solve_fail.ptr) h->solve_fail.ptr = host_words().take();
   CK(h->d_ticket.alloc(h->num_levels));
   CK(h->d_err.alloc(4));
   CK(h->d_inertia.alloc(2));
@@ -862,7 +871,7 @@ void run_solve(b200ldl_t h, int nrhs, double* x, int ldx) {
       sp.bdone = h->d_bdone.ptr;
       sp.epoch = h->solve_epoch;
       sp.fail = h->d_err.ptr + 3;
-      sp.host_fail = h->solve_fail;
+      sp.host_fail = h->solve_fail.ptr;
       sp.wait_polls = h->wait_polls;
       return sp;
     };
@@ -892,8 +901,8 @@ void run_solve(b200ldl_t h, int nrhs, double* x, int ldx) {
 void finish_solve(b200ldl_t h) {
   CK(cudaStreamSynchronize(h->stream));
   h->prof.collect();
-  if (h->solve_fail && *((volatile int*)h->solve_fail)) {
-    *h->solve_fail = 0;
+  if (h->solve_fail.ptr && *((volatile int*)h->solve_fail.ptr)) {
+    *h->solve_fail.ptr = 0;
     CK(cudaMemsetAsync(h->d_err.ptr + 3, 0, sizeof(int), h->stream));
     throw std::runtime_error("a supernode's neighbours were not solved in time");
   }
