@@ -95,7 +95,6 @@ struct Chain {
   int k, ncand;
   double *cur, *nx1, *nx2;  // the column at k, the next, the one after
   bool forced;  // the candidate at k is accepted as it stands
-  bool zero;    // and as a zero pivot: the other rows stay as they are
   bool moved;   // the column at k stands in cur alone (after a delay)
   int phase;    // which column barrier is next
   double thr, tol;  // a 1x1 passes with |d| >= tol and |d| >= thr max|column|
@@ -141,7 +140,7 @@ __device__ __forceinline__ void stage(double (&v)[kS][kR], Chain& h, const Front
     }
     const double d = cur[kD];
     const double absd = fabs(d);
-    const double r = (h.zero || (h.root && d == 0.0)) ? 0.0 : 1.0 / d;
+    const double r = (h.root && d == 0.0) ? 0.0 : 1.0 / d;
     if (!h.forced && !h.any) {
       // a bound of the lane's largest entry from its high word: a pivot that
       // passes against it passes (the rounded product is monotone), the full
@@ -150,7 +149,6 @@ __device__ __forceinline__ void stage(double (&v)[kS][kR], Chain& h, const Front
       if (!__all_sync(0xffffffffu, ok)) return;
     }
     h.forced = false;
-    h.zero = false;
     h.moved = false;
     const int nxt = k + 1;
     const bool more = nxt < h.ncand;
@@ -278,7 +276,7 @@ __device__ __forceinline__ Result factor_front(const Front& a, bool root, const 
   double* U = V + kLen;
   h.k = 0;
   h.ncand = a.fs;
-  h.forced = h.zero = h.moved = false;
+  h.forced = h.moved = false;
   h.phase = 0;
   h.thr = root ? kAlphaBK : prm.ustab;
   h.tol = root ? 0.0 : prm.pivot_tol;
@@ -364,6 +362,16 @@ __device__ __forceinline__ Result factor_front(const Front& a, bool root, const 
       a.orig[x] = a.orig[y];
       a.orig[y] = t;
     }
+  };
+
+  // the column at k is published and becomes the current one
+  auto next_column = [&]() {
+    if (k < ncand && warp == k % kWarps) publish(k, h.nx1);
+    double* t = h.cur;
+    h.cur = h.nx1;
+    h.nx1 = h.nx2;
+    h.nx2 = t;
+    __syncthreads();
   };
 
   if (k < ncand && warp == 0) publish(0, cur);
@@ -475,6 +483,30 @@ __device__ __forceinline__ Result factor_front(const Front& a, bool root, const 
       }
       continue;
     }
+    if (step == kZero && d != 0.0) {
+      // a zero pivot of a root whose diagonal is not a number, so that the
+      // reciprocal of stage() would not be zero: its column is zero, or not a
+      // number, which the products with zero keep
+      h.moved = false;
+      double w0[kR];
+#pragma unroll
+      for (int c = 0; c < kR; c++) {
+        const int i = lane + 32 * c;
+        w0[c] = (i > k && i < f) ? cur[i] : 0.0;
+        if (warp == k % kWarps && i > k && i < f) L[i + ld * k] = w0[c] * 0.0;
+      }
+      if (warp == k % kWarps && lane == 0) L[k + ld * k] = d;
+#pragma unroll
+      for (int s = 0; s < kS; s++) {
+        const int j = warp + kWarps * s;
+        const double x = (j > k && j < f) ? cur[j] * 0.0 : 0.0;
+#pragma unroll
+        for (int c = s / 4; c < kR; c++) v[s][c] = fma(-w0[c], x, v[s][c]);
+      }
+      k++;
+      next_column();
+      continue;
+    }
     if (step != kTwo) {
       if (kpiv != k) {
         replace(k, kpiv, cur);
@@ -489,7 +521,6 @@ __device__ __forceinline__ Result factor_front(const Front& a, bool root, const 
       // too, after an interchange).
       if (formed) __syncthreads();
       h.forced = true;
-      h.zero = step == kZero;
       continue;
     }
     // a 2x2 pivot: columns k and k + 1, with imax at k + 1
@@ -562,12 +593,7 @@ __device__ __forceinline__ Result factor_front(const Front& a, bool root, const 
     const int r = f - k - 2;
     out.flops += 2 * r * (r + 1) + 6 * r;
     k += 2;
-    if (k < ncand && warp == k % kWarps) publish(k, h.nx1);
-    double* t = h.cur;
-    h.cur = h.nx1;
-    h.nx1 = h.nx2;
-    h.nx2 = t;
-    __syncthreads();
+    next_column();
   }
   // a delayed candidate that was moved to k and stayed there
   if (h.moved && warp == k % kWarps) {
