@@ -32,6 +32,8 @@
 // Optimal control N = 1000 (167 supernodes of 64..68 rows one after another),
 // eight right-hand sides: 11.9 ms with a launch per level and sweep, 3.1 ms
 // now; one right-hand side of 512 such systems: 9.8 and 2.8 ms.
+#include <algorithm>
+
 #include "ldl_internal.h"
 #include "solve_common.cuh"
 
@@ -627,15 +629,24 @@ __global__ void __launch_bounds__(kSolveThreads, 2)
 constexpr size_t kSolveSmemMax = 224 * 1024;
 
 // doubles for the factor columns of a supernode: two diagonal blocks at
-// least; those of a 68-row front with 64 pivots where two CTAs per SM still
-// fit
+// least (stage_doubles)
 constexpr int kStageMin = 2 * kBlk * kTileLd;
-constexpr int kStageMax = 69 * 68;
 
 size_t solve_smem(int fmax, int nr, int stage_cap) {
   const int ld = nr == 1 ? 1 : nr == 2 ? 2 : nr <= 4 ? kVld<4> : kVld<8>;
   return (stage_cap + (size_t)ld * fmax) * sizeof(double) +
          (2 * (size_t)fmax + fmax / 31 + 4) * sizeof(int);
+}
+
+// Room for the factor columns in a launch of fronts up to fmax rows: all of
+// the largest front's, but at most 40 KB, so that two CTAs per SM (as many as
+// the registers allow) leave more than half of the SM's memory to L1, where
+// the fronts that do not fit are read; where two CTAs would not fit with that,
+// the two diagonal blocks.
+int stage_doubles(int fmax, int nr) {
+  const size_t most = 40 * 1024 / sizeof(double);
+  const int all = (int)std::min((size_t)(fmax | 1) * fmax, most);
+  return solve_smem(fmax, nr, all) <= 112 * 1024 ? std::max(kStageMin, all) : kStageMin;
 }
 
 }  // namespace
@@ -684,7 +695,7 @@ void launch_solve(const DevPlan& p, const DevState& s, const SolveSpan& sp, int 
   a.upool = upool;
   auto* k = nr == 1 ? solve_kernel<1> : nr == 2 ? solve_kernel<2> : nr <= 4 ? solve_kernel<4>
                                                                              : solve_kernel<8>;
-  a.stage_cap = solve_smem(sp.fmax, nr, kStageMax) <= 112 * 1024 ? kStageMax : kStageMin;
+  a.stage_cap = stage_doubles(sp.fmax, nr);
   k<<<sp.grid, kSolveThreads, solve_smem(sp.fmax, nr, a.stage_cap), stream>>>(p, s, a);
 }
 
