@@ -638,7 +638,7 @@ void run_factor_once(b200ldl_t h, const double* vals, const double* diag, bool m
       // its kernel variant (its CTAs per SM count there: 80,000 leaves of the
       // 256 x 256 plane-stress tree with the variant of larger fronts cost
       // 2.5 ms more than a launch saves).
-      constexpr int kFill = 148 * 4;
+      constexpr int kFill = kSMs * 4;
       int l1 = l + 1, fcap = h->level_fcap[l], width = h->level_ptr[l + 1] - b;
       if (!h->level_big[l])
         for (; l1 < h->num_levels && !h->level_big[l1]; l1++) {
@@ -865,7 +865,7 @@ void run_solve(b200ldl_t h, int nrhs, double* x, int ldx) {
       sp.count = big ? r.big_count : r.count;
       sp.fmax = big ? r.big_fmax : r.fmax;
       sp.ticket = (r.levels > 1 || both) ? h->d_solve_ticket.ptr + ticket : nullptr;
-      sp.grid = sp.ticket ? std::min({sp.count, 2 * r.width, 148 * 4}) : sp.count;
+      sp.grid = sp.ticket ? std::min({sp.count, 2 * r.width, kSMs * 4}) : sp.count;
       sp.parent = h->d_parent.ptr;
       sp.fdone = h->d_fdone.ptr;
       sp.bdone = h->d_bdone.ptr;

@@ -256,7 +256,7 @@ int b200ldl_assembly_values(b200ldl_assembly_t a, const double* blocks, double* 
   if (st != 0) return st;
   const int threads = 256;
   const int per_cta = threads * kPer;
-  const int grid = std::max(1, std::min((a->nnz - 1) / per_cta + 1, 148 * 64));
+  const int grid = std::max(1, std::min((a->nnz - 1) / per_cta + 1, b200ldl::kSMs * 64));
   const cudaStream_t st_ = static_cast<cudaStream_t>(stream);
   if (a->narrow)
     csr_gather_kernel<<<grid, threads, 0, st_>>>(a->nnz, a->d_ptr32.ptr, a->d_src32.ptr, blocks,

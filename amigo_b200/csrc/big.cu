@@ -891,7 +891,7 @@ cudaError_t assemble_big(const DevPlan& p, const DevState& s, const int* list, i
                                                                                         list);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  if (nl >= 148)
+  if (nl >= kSMs)
     e = launch_assemble_cl<1>(p, s, list, nl, vals, diag, stream);
   else if (nl >= 37)
     e = launch_assemble_cl<4>(p, s, list, nl, vals, diag, stream);
@@ -912,7 +912,7 @@ cudaError_t run_big_panels(const DevState& s, const FactorParams& prm, const int
   int NB = kBigPanelMax;
   while (NB > 4 && (size_t)R * (2 * (NB + 1) + 2) * sizeof(double) > kPanelSmemMax) NB >>= 1;
   const size_t smem = (size_t)R * (2 * (NB + 1) + 2) * sizeof(double);
-  const int upd_grid = 148 * 4;
+  const int upd_grid = kSMs * 4;
   const int cnb = big_chain_panel_width(max_f);
   const bool chained = cnb > 0;
   const int nsteps = chained ? (max_left + cnb - 2) / (cnb - 1) + 1

@@ -11,6 +11,8 @@ struct b200ldl_assembly;  // the assembly plan of the C ABI (assembly.cu)
 
 namespace b200ldl {
 
+constexpr int kSMs = 148;  // of a B200
+
 // Work counters accumulated on the device per factorization.
 constexpr int kWork = 8;
 

@@ -157,7 +157,7 @@ __global__ void perturb_diag_kernel(int n, const double* __restrict__ diag,
 void launch_perturb_diag(int n, const double* diag, const unsigned char* cls, double dx,
                          double dc, double* out, cudaStream_t st) {
   const int threads = 256;
-  const int blocks = std::max(1, std::min((n + threads - 1) / threads, 148 * 8));
+  const int blocks = std::max(1, std::min((n + threads - 1) / threads, kSMs * 8));
   perturb_diag_kernel<<<blocks, threads, 0, st>>>(n, diag, cls, dx, dc, out);
 }
 
