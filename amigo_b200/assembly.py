@@ -6,8 +6,8 @@ component group's elements, in order, add their Hessian columns into the
 fixed CSR pattern (ComponentGroup::add_hessian_kernel,
 include/component_group.h:144-162, CSRMat::add_row,
 include/csr_matrix.h:554-567). The library inverts that scatter once per
-pattern and sums every CSR entry's contributions in the reference's order
-with one thread per entry. The values are therefore bit-identical to the
+pattern and sums every CSR entry's contributions in the reference's order, by
+one thread (which takes two entries). The values are therefore bit-identical to the
 reference's CPU assembly and need no atomics (the reference's GPU backend
 uses atomicAdd). The result stays on the device and feeds
 ``SparseLDL.factor``.

@@ -212,10 +212,10 @@ struct b200ldl_handle {
   double exec_flops = 0.0;
   int fmax = 0;
   std::vector<int> level_fmax;
-  // solve schedule of the last factorization: per level, the supernodes for
-  // the one-CTA kernels then those for the cluster kernels
-  // of consecutive levels, the supernodes for the one-CTA kernel (from
-  // `first` on), then the last of these levels' for the cluster kernels
+  // Solve schedule of the last factorization, one run of consecutive levels
+  // after another: the run's supernodes for the one-CTA kernel (`count` of
+  // d_solve_nodes from `first` on), then those for the cluster kernels, which
+  // only the last of its levels has.
   struct SolveRun {
     int first = 0, count = 0, fmax = 1, width = 0, levels = 0;
     int big_count = 0, big_fmax = 1;

@@ -1426,7 +1426,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int i = tid; i < nl; i += kThreads) front_place(s, s.big[list[i]], info[i]);
   int step = 1;
   for (; step <= max_steps; step++) {
-    // ---- D: one warp per front
+    // ---- D: a warp factors the front's block; its CTA applies the delays
+    // where the level has no more fronts than CTAs, else the warp
     {
       WarpDiag& w = reinterpret_cast<WarpDiag*>(dsm)[warp];
       WarpDiag& w0 = reinterpret_cast<WarpDiag*>(dsm)[0];

@@ -234,15 +234,16 @@ __device__ __forceinline__ void run_stage(double (&v)[kS][kR], Chain& h, const F
 // the reciprocal itself, so that no decision has to travel; the warp that
 // owns the next column updates that column first and publishes it, and
 // arrives at the barrier before it goes on to its other columns. One barrier
-// and one shared-memory round trip per pivot: about 740 cycles a pivot for a
-// 68-row front with the code in the instruction cache, against about 2,800
-// for the same algorithm in shared memory with a reduction and a barrier per
-// pivot (optimal control N = 1000, 167 such fronts one after another: 17.0 ms
-// before, 7.2 ms now, launches included; 512 systems of 50..400 nodes: 13.3
-// and 7.5 ms). The other cases (statistics,
-// imax column, delays, interchanges, 2x2) are also decided by every warp from
-// the same values; an interchange moves two rows and columns between the
-// registers through the published columns.
+// and one shared-memory round trip per pivot: 0.4 us a pivot for a 68-row
+// front (740 cycles with the code in the instruction cache), against about
+// 2,800 cycles for the same algorithm in shared memory with a reduction and a
+// barrier per pivot. Optimal control N = 1000, 167 such fronts one after
+// another: 17.0 ms with that one and a launch per level, 7.0 ms now (42 us a
+// front, of which the pivots are 26: the rest is the way from one front to
+// the next). 512 systems of 50..400 nodes with 6 states: 13.3 and 7.4 ms. The
+// other cases (statistics, imax column, delays, interchanges, 2x2) are also
+// decided by every warp from the same values; an interchange moves two rows
+// and columns between the registers through the published columns.
 //
 // `write` is called with the number of pivots and then the trailing columns
 // (every lane's rows of its warp's columns) are handed to `store`.
