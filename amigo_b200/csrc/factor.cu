@@ -591,7 +591,7 @@ __global__ void __launch_bounds__(kFactorThreads, kMax == 1 ? 4 : kMax == 2 ? 3 
       fr.fs = fs;
       fr.ld = f | 1;
       fr.vec = fr.F + (size_t)fr.ld * f;
-      fr.fv = reinterpret_cast<int*>(fr.vec + 5 * vec_len(f));
+      fr.fv = reinterpret_cast<int*>(fr.vec + kVecs * vec_len(f));
       fr.orig = fr.fv + f;
       pos = reinterpret_cast<int*>(fr.vec);
       // a thread per own variable for the diagonal: two dependent loads each
@@ -788,7 +788,7 @@ size_t factor_smem_bytes(int f) {
   // the front (ld = f | 1), the travelling columns, the variables and their
   // positions at assembly
   const size_t ld = (size_t)(f | 1);
-  return (ld * f + 5 * (size_t)vec_len(f)) * sizeof(double) + 2 * (size_t)f * sizeof(int);
+  return (ld * f + kVecs * (size_t)vec_len(f)) * sizeof(double) + 2 * (size_t)f * sizeof(int);
 }
 
 namespace {

@@ -69,7 +69,7 @@ __device__ __forceinline__ double two_products(double a, double b, double c, dou
 // The front of one CTA: assembled in shared memory, factored in registers.
 struct Front {
   double* F;     // [f][ld], column-major lower triangle, then the factor columns
-  double* vec;   // [5][vec_len(f)] columns that travel between the warps
+  double* vec;   // [kVecs][vec_len(f)] columns that travel between the warps
   int* fv;       // [f] front variables in the current order
   int* orig;     // [f] their positions at assembly
   int f, fs, ld;
@@ -89,6 +89,8 @@ __host__ __device__ __forceinline__ int row_chunks(int f) {
 // for the others from its chunk on (so that no reader has to compare rows),
 // and the diagonal entry after the last chunk.
 __host__ __device__ __forceinline__ int vec_len(int f) { return 32 * row_chunks(f) + 2; }
+
+constexpr int kVecs = 6;  // of them
 
 // Where the pivot chain stands, the same in every warp.
 struct Chain {
@@ -267,14 +269,15 @@ __device__ __forceinline__ Result factor_front(const Front& a, bool root, const 
     }
   }
   // the current column, the next one, the one after (a warp may still read
-  // the current one when the next but one is published), and two for the
-  // imax column and the interchanges
+  // the current one when the next but one is published), two for the imax
+  // column and the interchanges, and the next candidate's imax column
   Chain h;
   h.cur = a.vec;
   h.nx1 = h.cur + kLen;
   h.nx2 = h.nx1 + kLen;
   double* V = h.nx2 + kLen;
   double* U = V + kLen;
+  double* spare = U + kLen;
   h.k = 0;
   h.ncand = a.fs;
   h.forced = h.moved = false;
@@ -517,10 +520,15 @@ __device__ __forceinline__ Result factor_front(const Front& a, bool root, const 
         V = t;
       }
       // In the stage the next column's warp only arrives at the barrier. If
-      // its column does not pass either it goes on to form another row in V,
-      // which the other warps must have read by then (the old current column
-      // too, after an interchange).
-      if (formed) __syncthreads();
+      // its column does not pass either it goes on to form another row while
+      // other warps may still read V (the old current column, after an
+      // interchange): that row goes into the spare, and the barrier after it
+      // is what lets V be formed in again.
+      if (formed) {
+        double* t = V;
+        V = spare;
+        spare = t;
+      }
       h.forced = true;
       continue;
     }

@@ -349,7 +349,7 @@ extern "C" int front_schedules(int chunks, int f, int fs, int root, int cholesky
   for (int i = 0; i < f; i++) result[4] += wo[i] != i;
   const double nan = std::nan("");
   for (unsigned how = first; how < first + count; how++) {
-    std::vector<double> mem((size_t)ld * f + 5 * len + 2 * guard, nan);
+    std::vector<double> mem((size_t)ld * f + kVecs * len + 2 * guard, nan);
     std::vector<double> got((size_t)f * f, 0.0);
     std::vector<int> fv(f), orig(f);
     Front fr;
@@ -373,7 +373,7 @@ extern "C" int front_schedules(int chunks, int f, int fs, int root, int cholesky
       if (threadIdx.x == 0) r = q;
     };
     const char* bad = sim::run(s, how);
-    const double* end = fr.vec + 5 * len;
+    const double* end = fr.vec + kVecs * len;
     for (int i = 0; i < guard && !bad; i++)
       if (!std::isnan(mem[i]) || !std::isnan(end[i])) bad = "a write out of range";
     if (!bad && (r.npiv != w.npiv || r.npos != w.npos || r.nneg != w.nneg || r.flops != w.flops))
