@@ -240,9 +240,9 @@ __device__ __forceinline__ void run_stage(double (&v)[kS][kR], Chain& h, const F
 // front (740 cycles with the code in the instruction cache), against about
 // 2,800 cycles for the same algorithm in shared memory with a reduction and a
 // barrier per pivot. Optimal control N = 1000, 167 such fronts one after
-// another: 17.0 ms with that one and a launch per level, 7.0 ms now (42 us a
+// another: 17.0 ms with that one and a launch per level, 6.9 ms now (41 us a
 // front, of which the pivots are 26: the rest is the way from one front to
-// the next). 512 systems of 50..400 nodes with 6 states: 13.3 and 7.4 ms. The
+// the next). 512 systems of 50..400 nodes with 6 states: 13.3 and 7.3 ms. The
 // other cases (statistics, imax column, delays, interchanges, 2x2) are also
 // decided by every warp from the same values; an interchange moves two rows
 // and columns between the registers through the published columns.

@@ -30,7 +30,7 @@
 // the factor), and wait for the children's flags (forward) or the parent's
 // (backward). Both sweeps share a launch when no supernode needs a cluster.
 // Optimal control N = 1000 (167 supernodes of 64..68 rows one after another),
-// eight right-hand sides: 11.9 ms with a launch per level and sweep, 3.1 ms
+// eight right-hand sides: 11.9 ms with a launch per level and sweep, 3.2 ms
 // now; one right-hand side of 512 such systems: 9.8 and 2.8 ms.
 #include <algorithm>
 
